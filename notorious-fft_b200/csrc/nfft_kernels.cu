@@ -1,7 +1,7 @@
 // nfft_kernels.cu -- instantiation and launch of the pass kernels, the
 // unpack epilogue, the size-1 kernel, and the plan-time kernels (twiddle
 // tables from FP64 sincospi; Bluestein chirp from exact k^2 mod 2n).
-#include "nfft_engine.h"
+#include "nfft_blue.h"
 
 #include <atomic>
 
@@ -12,47 +12,28 @@ static std::atomic<long long> g_launches{0};
 long long launch_count() { return g_launches.load(); }
 void note_launch() { g_launches++; }
 
+// Generic pass kernels (nfft_pass_slice.cuh, compiled in slices).
 using PassFn = void (*)(const PassArgs);
-
-// Valid (load, store) operator pairs.  Others are never planned.
-#define NFFT_PAIRS(X)          \
-    X(LD_C, ST_C)              \
-    X(LD_C, ST_R)              \
-    X(LD_C, ST_T2)             \
-    X(LD_C, ST_T3)             \
-    X(LD_C, ST_T4)             \
-    X(LD_C, ST_BLUE)           \
-    X(LD_T2, ST_C)             \
-    X(LD_T2, ST_T2)            \
-    X(LD_T3, ST_C)             \
-    X(LD_T3, ST_T3)            \
-    X(LD_IR, ST_C)             \
-    X(LD_T4, ST_C)             \
-    X(LD_T4, ST_T4)            \
-    X(LD_BLUE, ST_C)           \
-    X(LD_BLUE, ST_BLUE)        \
-    X(LD_R2C, ST_C)            \
-    X(LD_R2C, ST_R)            \
-    X(LD_C, ST_C2R)            \
-    X(LD_IR, ST_C2R)           \
-    X(LD_FILT, ST_C)
-
 constexpr int NLOAD = NUM_LOAD_OPS, NSTORE = NUM_STORE_OPS;
+struct PassTable {
+    PassFn t12[NLOAD][NSTORE] = {}, t13[NLOAD][NSTORE] = {};
+};
+void pass_register_slice_0(PassFn (*t12)[NUM_STORE_OPS], PassFn (*t13)[NUM_STORE_OPS]);
+void pass_register_slice_1(PassFn (*t12)[NUM_STORE_OPS], PassFn (*t13)[NUM_STORE_OPS]);
+void pass_register_slice_2(PassFn (*t12)[NUM_STORE_OPS], PassFn (*t13)[NUM_STORE_OPS]);
+void pass_register_slice_3(PassFn (*t12)[NUM_STORE_OPS], PassFn (*t13)[NUM_STORE_OPS]);
 
 static PassFn pass_table(int log_tile, int ld, int st) {
-    static PassFn t12[NLOAD][NSTORE] = {};
-    static PassFn t13[NLOAD][NSTORE] = {};
-    static bool filled = false;
-    if (!filled) {
-#define X(L, S)                                          \
-    t12[L][S] = pass_kernel<real_t, 12, L, S>;           \
-    t13[L][S] = pass_kernel<real_t, 13, L, S>;
-        NFFT_PAIRS(X)
-#undef X
-        filled = true;
-    }
+    static const PassTable tab = [] {
+        PassTable t;
+        pass_register_slice_0(t.t12, t.t13);
+        pass_register_slice_1(t.t12, t.t13);
+        pass_register_slice_2(t.t12, t.t13);
+        pass_register_slice_3(t.t12, t.t13);
+        return t;
+    }();
     if (ld < 0 || ld >= NLOAD || st < 0 || st >= NSTORE) return nullptr;
-    return log_tile == 13 ? t13[ld][st] : (log_tile == 12 ? t12[ld][st] : nullptr);
+    return log_tile == 13 ? tab.t13[ld][st] : (log_tile == 12 ? tab.t12[ld][st] : nullptr);
 }
 
 void lean_register_slice_0(LeanRegistry&);
@@ -101,6 +82,7 @@ bool launch_lean(const PassArgs& a, int logT, int ci, int co, int ld, int st, lo
 }
 
 bool set_kernel_attributes() {
+    if (!blue_set_attributes()) return false;
     for (auto& kv : lean_registry().entries) {
         if (!cuda_ok(cudaFuncSetAttribute(kv.second.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kv.second.smem),
                      "cudaFuncSetAttribute(lean pass)"))

@@ -6,6 +6,7 @@
 
 #include <algorithm>
 
+#include "nfft_blue.h"
 #include "nfft_engine.h"
 #include "nfft_queue.h"
 
@@ -440,6 +441,12 @@ bool run_pass(const DeviceCtx* c, const View& src, const View& dst, int logL, in
         rec->launches.push_back(r);
         return true;
     }
+    // whole Bluestein transforms of contiguous lines (1-D and last axes; the
+    // strided axes of N-D shapes keep the general kernel, whose column walk
+    // reads their unit-stride direction)
+    if (mid && ldop == LD_BLUE && stop == ST_BLUE && a.in_row && a.out_row && logR >= BLUE_MIN_LOGM &&
+        logR <= BLUE_MAX_LOGM && !lean_disabled())
+        return launch_blue(a, s);
     // split tensor-core form: radix-256 passes on tcgen05 where the layout
     // allows (unit-stride lines, aligned strides), else in the warp-level
     // specialized kernel; other radices with the radix-16 sub-stages of the

@@ -197,6 +197,7 @@ __host__ __device__ void nfft_emu_smem_check(int idx) {
 #include "../../notorious-fft_b200/csrc/nfft_queue_build.cu"
 #include "../../notorious-fft_b200/csrc/nfft_lean.cuh"
 #include "../../notorious-fft_b200/csrc/nfft_lean_list.h"
+#include "../../notorious-fft_b200/csrc/nfft_blue.cuh"
 #include "../../notorious-fft_b200/csrc/nfft_tc.cuh"
 #include "../../notorious-fft_b200/csrc/nfft_tc_lean.cuh"
 #include "../../notorious-fft_b200/csrc/nfft_umma.cuh"
@@ -454,6 +455,81 @@ static void emu_lean(const PassArgs& a, long long t0, long long t1) {
             for (int t = 0; t < TH; ++t) paired_unpack_thread<Lt, T, ST>(a, tw, sm.data(), lines.data(), t);
         }
     }
+}
+
+// ---- single-tile Bluestein kernels: the kernel body of nfft_blue.cuh
+template <int LOGM, int LOGT, int LD, int ST>
+static void emu_blue(const PassArgs& a, long long t0, long long t1) {
+    using T = real_t;
+    using V = C2<T>;
+    using B = Blue<T, LOGM, LOGT, LD, ST>;
+    const TwTables<T>* tw = (const TwTables<T>*)a.tw;
+    constexpr int TH = B::THREADS, NS = B::NS;
+    g_smem_elems = B::SMEM_ELEMS;
+    std::vector<V> sm(B::SMEM_ELEMS), regs((size_t)TH * 16);
+    std::vector<LeanLine> lines(B::J);
+    auto all = [&](auto f) {
+        for (int t = 0; t < TH; ++t) f(t, &regs[(size_t)t * 16]);
+    };
+    auto middle = [&](auto Sc, auto Ic) {
+        constexpr int S = decltype(Sc)::value;
+        constexpr bool INV = decltype(Ic)::value;
+        all([&](int t, V* v) { B::template read<S, INV>(sm.data(), t, v); });
+        all([&](int t, V* v) {
+            B::template dfts<S, INV>(tw, t, v);
+            B::template write<S, INV>(sm.data(), t, v);
+        });
+    };
+    for (long long tile = t0; tile < t1; ++tile) {
+        const long long line0 = tile << B::LOGJ;
+        if (line0 >= a.nlines) continue;
+        for (auto& x : sm) x = mkc((T)NAN, (T)NAN);
+        for (int t = 0; t < B::J; ++t) {
+            long long tmp[3];
+            line_setup(a, line0 + t, 0, TileLines{&tmp[0], &tmp[1], &tmp[2]});
+            lines[t] = LeanLine{tmp[0], tmp[1], tmp[2]};
+        }
+        all([&](int t, V* v) { B::load(a, lines.data(), t, v); });
+        if constexpr (NS >= 2) {
+            all([&](int t, V* v) { B::template write<0, false>(sm.data(), t, v); });
+            if constexpr (NS >= 3) middle(std::integral_constant<int, 1>{}, std::false_type{});
+            if constexpr (NS >= 4) middle(std::integral_constant<int, 2>{}, std::false_type{});
+            all([&](int t, V* v) {
+                B::template read<NS - 1, false>(sm.data(), t, v);
+                B::template dfts<NS - 1, false>(tw, t, v);
+            });
+        }
+        all([&](int t, V* v) { B::filter(a, t, v); });
+        if constexpr (NS >= 2) {
+            all([&](int t, V* v) { B::template write<0, true>(sm.data(), t, v); });
+            if constexpr (NS >= 3) middle(std::integral_constant<int, 1>{}, std::true_type{});
+            if constexpr (NS >= 4) middle(std::integral_constant<int, 2>{}, std::true_type{});
+            all([&](int t, V* v) {
+                B::template read<NS - 1, true>(sm.data(), t, v);
+                B::template dfts<NS - 1, true>(tw, t, v);
+            });
+        }
+        all([&](int t, V* v) { B::store(a, lines.data(), t, v); });
+    }
+}
+
+static long long g_blue_launches = 0;
+bool launch_blue(PassArgs a, cudaStream_t) {
+    static const EmuFn tab[] = {
+        emu_blue<4, blue_logt(4), LD_BLUE, ST_BLUE>,   emu_blue<5, blue_logt(5), LD_BLUE, ST_BLUE>,
+        emu_blue<6, blue_logt(6), LD_BLUE, ST_BLUE>,   emu_blue<7, blue_logt(7), LD_BLUE, ST_BLUE>,
+        emu_blue<8, blue_logt(8), LD_BLUE, ST_BLUE>,   emu_blue<9, blue_logt(9), LD_BLUE, ST_BLUE>,
+        emu_blue<10, blue_logt(10), LD_BLUE, ST_BLUE>, emu_blue<11, blue_logt(11), LD_BLUE, ST_BLUE>,
+        emu_blue<12, blue_logt(12), LD_BLUE, ST_BLUE>, emu_blue<13, blue_logt(13), LD_BLUE, ST_BLUE>};
+    if (a.logR < BLUE_MIN_LOGM || a.logR > BLUE_MAX_LOGM) {
+        set_error(6, "no Bluestein tile kernel for a padded length of 2^%d", a.logR);
+        return false;
+    }
+    a.logJ = blue_logt(a.logR) + 4 - a.logR;
+    g_launches++;
+    g_blue_launches++;
+    tab[a.logR - BLUE_MIN_LOGM](a, 0, (a.nlines + (1ll << a.logJ) - 1) >> a.logJ);
+    return true;
 }
 
 void note_launch() { g_launches++; }
@@ -1022,6 +1098,7 @@ void nfft_emu_unregister_host(void* p) {
 }
 long long nfft_emu_launches(void) { return nfft::g_launches; }
 long long nfft_emu_lean_launches(void) { return nfft::g_lean_launches; }
+long long nfft_emu_blue_launches(void) { return nfft::g_blue_launches; }
 long long nfft_emu_checks(void) { return emu::n_checks; }
 long long nfft_emu_queue_items(void) { return nfft::g_queue_items; }
 long long nfft_emu_umma_launches(void) { return nfft::g_umma_launches; }

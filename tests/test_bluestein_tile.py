@@ -1,0 +1,51 @@
+"""Single-tile Bluestein kernels: the shortest and longest length of every padded
+size, batches that end inside a tile, padded distances, both directions, in
+place; on the CPU emulator (bounds-checked) and on the GPU, against the oracle.
+Tolerance: the library's bars, 1e-13 log2 N (double) and 1e-6 log2 N (float).
+"""
+import math
+
+import numpy as np
+import pytest
+
+from oracle import rel_l2
+
+# (length, transforms): M = 16 .. 8192, tiles of 2048 points and one line above
+CASES = [(5, 257), (7, 3), (9, 130), (15, 1), (17, 33), (31, 65), (33, 17), (63, 2), (65, 9), (127, 8), (129, 5),
+         (255, 4), (257, 3), (511, 1), (513, 3), (1000, 2), (1025, 1), (2047, 2), (2049, 1), (4095, 2)]
+
+
+def check(lib, oracle, n, batch, put=lambda a: a, get=lambda a: a, device=False):
+    bar = (1e-6 if lib.single else 1e-13) * math.log2(n)
+    rng = np.random.default_rng(n)
+    x = (rng.uniform(-1, 1, (batch, n + 3)) + 1j * rng.uniform(-1, 1, (batch, n + 3))).astype(lib.cdt)
+    with lib.mkaux("dft", [n]) as a:
+        for kind in ("dft", "invdft"):
+            want = np.stack([oracle.transform(kind, r) for r in x[:, :n].astype(complex)])
+            y = put(np.zeros((batch, n + 1), lib.cdt))
+            a.batched(kind, put(x), y, batch, n + 3, n + 1)
+            assert rel_l2(get(y)[:, :n], want) <= bar, kind
+            z = put(x.copy())
+            a.batched(kind, z, z, batch, n + 3, n + 3)
+            assert rel_l2(get(z)[:, :n], want) <= bar, kind + " in place"
+            if device:   # host arrays are staged whole
+                assert np.array_equal(get(z)[:, n:], x[:, n:]), "stores outside the lines"
+
+
+@pytest.mark.parametrize("n,batch", CASES)
+@pytest.mark.parametrize("single", [False, True])
+def test_emulated(emu_d, emu_f, oracle_d, n, batch, single):
+    check(emu_f if single else emu_d, oracle_d, n, batch)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,batch", CASES)
+@pytest.mark.parametrize("single", [False, True])
+def test_gpu(lib_d, lib_f, oracle_d, n, batch, single):
+    import torch
+
+    def get(t):
+        torch.cuda.synchronize()
+        return t.cpu().numpy()
+
+    check(lib_f if single else lib_d, oracle_d, n, batch, lambda a: torch.from_numpy(a).cuda(), get, True)
