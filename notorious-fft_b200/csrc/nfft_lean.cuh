@@ -127,17 +127,21 @@ struct Lean {
     // paired stores need whole lines in the tile: row tiles, or mirror tiles
     // (column in and out) for the last pass of a multi-pass transform
     static constexpr bool MIRROR = PAIRED && COL_IN && COL_OUT;
-    // row tile of a single-pass DCT-3 / DST-3 or inverse real transform: the
-    // input repack runs as a paired phase into shared memory
-    // (pair_prepack_thread) and the first sub-stage reads its points from there
-    static constexpr bool PREPACK = (LOAD == LD_T3 || LOAD == LD_IR) && !COL_IN;
+    // DCT-3 / DST-3 and inverse real transforms: the input repack runs as a
+    // paired phase into shared memory (pair_prepack_thread) and the first
+    // sub-stage reads its points from there.  Row tiles hold whole lines; the
+    // first pass of a multi-pass transform (column in, row out) pairs line j
+    // with line ns - j in the tile, like the mirror tiles of the last pass.
+    static constexpr bool PREPACK = LOAD == LD_T3 || LOAD == LD_IR;
+    static constexpr bool MIRROR_IN = PREPACK && COL_IN;
+    static_assert(!(MIRROR_IN && (COL_OUT || LOGJ < 1)), "the repacking pass of multi-pass transforms writes rows");
     static_assert(!(PAIRED && (COL_IN != COL_OUT)), "paired operators need row tiles or mirror tiles");
     static_assert(!MIRROR || LOGJ >= 1, "mirror tiles pair lines");
 
     // first sub-stage (points from shared memory, then the radix-16 DFT) of PREPACK tiles
     static NFFT_HD void first_smem(const PassArgs& a, const TwTables<T>* tw, const C2<T>* sm, const LeanLine* lines,
                                    int t, C2<T>* v, int& l, int& i) {
-        lean_map<false, LOGJ>(t, LOGR - 4, l, i);
+        lean_map<COL_IN, LOGJ>(t, LOGR - 4, l, i);
         const LeanLine ln = lines[l];
         if (ln.j < 0) {
 #pragma unroll
@@ -145,7 +149,7 @@ struct Lean {
             return;
         }
 #pragma unroll
-        for (int m = 0; m < 16; ++m) v[m] = sm[NFFT_SM((lean_idx<false, LOGR, LOGJ>(l, i + (m << (LOGR - 4)))))];
+        for (int m = 0; m < 16; ++m) v[m] = sm[NFFT_SM((lean_idx<COLL, LOGR, LOGJ>(l, i + (m << (LOGR - 4)))))];
         pre_twiddle_dft(a, tw, ln.j, i, v);
     }
 
@@ -563,73 +567,149 @@ NFFT_HD void paired_unpack_thread(const PassArgs& a, const TwTables<T>* tw, cons
     }
 }
 
-// Paired input repack of a row tile (PREPACK): the inverse-real repack
+// Paired input repack (PREPACK): the inverse-real repack
 // p -> conj(s + i e^{+2 pi i p/N} d), s / d from the bins z_p and conj z_{M-p},
 // for invrealdft (z = the input bins; bins 1 .. M-1 halved for the adjoint of
 // realdft) and DCT-3 / DST-3 (z = the pre-twiddled reorder zb of the reals;
-// zb_0 doubled for the adjoint of DCT-2 / DST-2).  Item (l, k), k = 0 .. M/2,
-// of the tile's lines takes z_k and z_{M-k} once and writes points k and M - k
-// of line l (W_N^{M-k} = -conj W_N^k and e^{-i pi (M-k)/2N} = e^{-i pi/4}
-// conj e^{-i pi k/2N} exactly), where the generic operators compute both
-// members of a pair for each point; items walk k fastest so neighbouring
-// threads read neighbouring points.
+// zb_0 doubled for the adjoint of DCT-2 / DST-2).  An item is a pair of bins k,
+// M - k: it takes z_k and z_{M-k} once and writes both points
+// (W_N^{M-k} = -conj W_N^k and e^{-i pi (M-k)/2N} = e^{-i pi/4} conj
+// e^{-i pi k/2N} exactly), where the generic operators compute both members of
+// a pair for each point.  Every thread has 8 items; all their loads are issued
+// before any is used, and their twiddles are one table root each times exact
+// roots of order <= 4096, so an item costs one product more than a lookup.
+// Row tiles: items walk k along a line.  Mirror-in tiles: item (l, r) is bin
+// j + r ns of the low line j and its partner, point R - 1 - r of line ns - j;
+// the first low line of a transform's first tile (j = 0) and its high line
+// (j = ns / 2) pair with themselves (mirror_item_k).  Items walk lines fastest.
+// Bound by HBM like a plain pass.  B200, before (a loop of dependent loads; the
+// first pass of several through the generic operator) -> now: invrealdft 2^20 x
+// 16 FP64 230 -> 180 us, DCT-3 2^18 x 81 FP64 390 -> 245 us, realdft + invrealdft
+// 32768 x 512 FP32 90 -> 75 us, 4096 x 2000 FP64 97 -> 80 us.
 template <typename L, typename T, int LOAD>
-NFFT_HD void pair_prepack_thread(const PassArgs& a, const TwTables<T>* tw, C2<T>* sm, const LeanLine* lines, int t) {
+NFFT_HD void pair_prepack_thread(const PassArgs& a, const TwTables<T>* tw, C2<T>* sm, const LeanLine* lines,
+                                 long long tile, int t) {
     using V = C2<T>;
-    constexpr int LOGR = L::LOGR_;
-    constexpr int M = 1 << LOGR;
-    constexpr int NI = M / 2 + 1;   // items per line
-    const long long N = 2ll * M, es = a.in_estride;
+    constexpr int LOGR = L::LOGR_, R = 1 << LOGR, NI = 8;
+    constexpr bool MIR = L::MIRROR_IN;
+    constexpr int H = MIR ? L::J / 2 : R / 2;   // low lines of a tile / items of a line
+    static_assert(MIR ? H * R == NI * L::THREADS : L::J * H == NI * L::THREADS, "8 items per thread");
+    const long long es = a.in_estride;
+    const long long ns = MIR ? 1ll << a.logNj : 1;
+    const long long M = ns << LOGR, N = 2 * M;
+    auto put = [&](int l, int r, V v) { sm[NFFT_SM((lean_idx<L::COLL, LOGR, L::LOGJ>(l, r)))] = v; };
+    // first tile of a transform, first low line: self-paired lines
+    bool self = false;
+    if constexpr (MIR) self = tile % (ns >> L::LOGJ) == 0 && (t & (H - 1)) == 0;
+    // item q: local lines and points of bins k and M - k, and k
+    auto item = [&](int q, int& lA, int& rA, int& lB, int& rB) -> long long {
+        const int w = t + q * L::THREADS;
+        if constexpr (MIR) {
+            const int l = w & (H - 1), r = w / H;
+            if (!self) {
+                lA = l; rA = r; lB = H + l; rB = R - 1 - r;
+                return lines[l].j + r * ns;
+            }
+            if (r < R / 2) {
+                lA = lB = 0; rA = r; rB = R - r;
+                return r * ns;
+            }
+            lA = lB = H; rA = r - R / 2; rB = R - 1 - rA;
+            return ns / 2 + rA * ns;
+        } else {
+            lA = lB = w / H; rA = w & (H - 1); rB = R - rA;
+            return rA;
+        }
+    };
+    // the two bins of pair k as raw input values: zk, zm (LD_IR), or the reals
+    // (x_k, x_{N-k}), (x_{M-k}, x_{M+k}) behind zb_k and zb_{M-k} (LD_T3)
+    auto raw = [&](long long base, long long k, V& u, V& v) {
+        if constexpr (LOAD == LD_IR) {
+            const V* z = (const V*)a.in + base;
+            u = NFFT_GLD(&z[k * es]);
+            v = NFFT_GLD(&z[(M - k) * es]);
+        } else {
+            const T* x = (const T*)a.in + base;
+            const long long iA = a.dst ? N - 1 - k : k, iB = k == 0 ? iA : (a.dst ? k - 1 : N - k);
+            const long long iC = a.dst ? M - 1 + k : M - k, iD = a.dst ? M - 1 - k : M + k;
+            u = mkc(NFFT_GLD(&x[iA * es]), NFFT_GLD(&x[iB * es]));
+            v = mkc(NFFT_GLD(&x[iC * es]), NFFT_GLD(&x[iD * es]));
+        }
+    };
+    auto pre = [&](V x, V tq) { return mkc(x.x * tq.x - x.y * tq.y, -x.x * tq.y - x.y * tq.x); };
     auto rep = [](V u, V v2, V w2) {
         const V b = cconj(v2);
         const V s2 = cadd(u, b), d = csub(u, b);
         const V od = cmulc(d, w2);
         return cconj(mkc(s2.x - od.y, s2.y + od.x));
     };
-    for (int w = t; w < L::J * NI; w += L::THREADS) {
-        const int l = w / NI, k = w - l * NI;
-        const LeanLine ln = lines[l];
-        auto put = [&](int p, V val) { sm[NFFT_SM((lean_idx<false, LOGR, L::LOGJ>(l, p)))] = val; };
-        if (ln.j < 0) {
-            put(k, mkc((T)0, (T)0));
-            if (k > 0 && k < M / 2) put(M - k, mkc((T)0, (T)0));
-            continue;
+    V u[NI], v[NI], uh = V{}, vh = V{};
+    // bin M / 2 pairs with itself: one per line (row tiles) or transform
+    const bool half = MIR ? self && t < H : t < L::J && lines[t].j >= 0;
+#pragma unroll
+    for (int q = 0; q < NI; ++q) {
+        int lA, rA, lB, rB;
+        const long long k = item(q, lA, rA, lB, rB);
+        const LeanLine ln = lines[lA];
+        if (ln.j >= 0) raw(ln.bin, k, u[q], v[q]);
+        else u[q] = v[q] = mkc((T)0, (T)0);
+    }
+    if (half) raw(lines[MIR ? 0 : t].bin, M / 2, uh, vh);
+    // twiddles: bins of a thread step by 1 (row tiles, within a line) or D ns
+    V w0 = V{}, t0 = V{};
+    constexpr int D = MIR ? L::THREADS / H : 1;
+    {
+        int lA, rA, lB, rB;
+        const long long k0 = item(0, lA, rA, lB, rB);
+        w0 = twiddle<T>(tw, (uint64_t)k0, a.logN);
+        if constexpr (LOAD == LD_T3) t0 = twiddle<T>(tw, (uint64_t)k0, a.logN + 2);
+    }
+#pragma unroll
+    for (int q = 0; q < NI; ++q) {
+        int lA, rA, lB, rB;
+        const long long k = item(q, lA, rA, lB, rB);
+        V wk = w0, tk = t0;
+        if constexpr (MIR) {
+            if (self) {
+                wk = twiddle<T>(tw, (uint64_t)k, a.logN);
+                if constexpr (LOAD == LD_T3) tk = twiddle<T>(tw, (uint64_t)k, a.logN + 2);
+            } else if (q > 0) {   // W_N^{q D ns} = W_{2R}^{q D}, e^{-i pi q D ns / 2N} = W_{8R}^{q D}
+                wk = cmul(w0, twiddle<T>(tw, (uint64_t)(q * D), LOGR + 1));
+                if constexpr (LOAD == LD_T3) tk = cmul(t0, twiddle<T>(tw, (uint64_t)(q * D), LOGR + 3));
+            }
+        } else if constexpr (H > L::THREADS) {
+            constexpr int PER = H / L::THREADS, LT = L::LOGTILE - 4;
+            if (q % PER) {        // k = t + (q mod PER) THREADS
+                wk = cmul(w0, twiddle_small<T>(tw, (uint32_t)(q % PER), LOGR + 1 - LT));
+                if constexpr (LOAD == LD_T3) tk = cmul(t0, twiddle_small<T>(tw, (uint32_t)(q % PER), LOGR + 3 - LT));
+            }
         }
-        V zk, zm;
+        V zk = u[q], zm = v[q];
         if constexpr (LOAD == LD_IR) {
-            const V* z = (const V*)a.in + ln.bin;
-            zk = NFFT_GLD(&z[k * es]);
-            zm = NFFT_GLD(&z[(M - k) * es]);
             if (a.vjp && k > 0) {
                 zk = cscale(zk, (T)0.5);
                 zm = cscale(zm, (T)0.5);
             }
         } else {
-            const T* x = (const T*)a.in + ln.bin;
-            if (k == 0) {
-                zk = mkc(NFFT_GLD(&x[(a.dst ? N - 1 : 0) * es]), (T)0);
-                zm = mkc((T)K<T>::r2 * (T)2 * NFFT_GLD(&x[(a.dst ? M - 1 : M) * es]), (T)0);
-                if (a.vjp) zk = cscale(zk, (T)2);
-            } else {
-                const V tk = twiddle<T>(tw, (uint64_t)k, LOGR + 3);   // e^{-i pi k / 2N}
-                const V tm = mkc((tk.x - tk.y) * K<T>::r2, -(tk.x + tk.y) * K<T>::r2);
-                auto zb = [&](long long q, V tq) -> V {
-                    const T xr = a.dst ? NFFT_GLD(&x[(N - q - 1) * es]) : NFFT_GLD(&x[q * es]);
-                    const T xi = a.dst ? NFFT_GLD(&x[(q - 1) * es]) : NFFT_GLD(&x[(N - q) * es]);
-                    return mkc(xr * tq.x - xi * tq.y, -xr * tq.y - xi * tq.x);
-                };
-                zk = zb(k, tk);
-                zm = zb(M - k, tm);
-            }
+            if (k == 0) zk = mkc(a.vjp ? (T)2 * zk.x : zk.x, (T)0);
+            else zk = pre(zk, tk);
+            zm = pre(zm, mkc((tk.x - tk.y) * K<T>::r2, -(tk.x + tk.y) * K<T>::r2));
         }
         if (k == 0) {
-            put(0, cconj(mkc(zk.x + zm.x, zk.x - zm.x)));
-            continue;
+            put(lA, 0, mkc(zk.x + zm.x, zm.x - zk.x));
+        } else {
+            put(lA, rA, rep(zk, zm, wk));
+            put(lB, rB, rep(zm, zk, mkc(-wk.x, wk.y)));
         }
-        const V wk = twiddle<T>(tw, (uint64_t)k, LOGR + 1);   // W_N^k
-        put(k, rep(zk, zm, wk));
-        if (k < M / 2) put(M - k, rep(zm, zk, mkc(-wk.x, wk.y)));
     }
+    if (half) {
+        // p = M / 2: z pairs with itself and W_N^p = -i, so the point is 2 z
+        V z = uh;
+        if constexpr (LOAD == LD_IR) z = cscale(z, a.vjp ? (T)1 : (T)2);
+        else z = cscale(pre(z, mkc(K<T>::c8, -K<T>::s8)), (T)2);
+        put(MIR ? 0 : t, R / 2, z);
+    }
+    (void)vh;
 }
 
 // One tile of a specialized pass (all threads of the CTA call it; uniform
@@ -647,7 +727,7 @@ __device__ __forceinline__ void lean_tile(const PassArgs& a, long long tile, uns
     if (t < L::J) {
         long long tmp[3];
         TileLines tl{&tmp[0], &tmp[1], &tmp[2]};
-        if constexpr (L::MIRROR) {
+        if constexpr (L::MIRROR || L::MIRROR_IN) {
             const long long ns = 1ll << a.logNj, tpt = ns >> L::LOGJ;   // lines, tiles per transform
             const long long tr = tile / tpt, tt = tile - tr * tpt;
             line_setup(a, tr * ns + mirror_line(tt, t, L::J, ns), 0, tl);
@@ -661,7 +741,7 @@ __device__ __forceinline__ void lean_tile(const PassArgs& a, long long tile, uns
     V v[16];
     int l, i;
     if constexpr (L::PREPACK) {
-        pair_prepack_thread<L, T, LOAD>(a, tw, sm, lines, t);
+        pair_prepack_thread<L, T, LOAD>(a, tw, sm, lines, tile, t);
         __syncthreads();
         L::first_smem(a, tw, sm, lines, t, v, l, i);
         __syncthreads();   // every point read before the sub-stage writes

@@ -478,7 +478,10 @@ bool run_pass(const DeviceCtx* c, const View& src, const View& dst, int logL, in
             (rr || 7 + 4 - logR >= log_jmin()))
             logT = 7;
         if (op.logt && lean_available(logR, op.logt, ci, co, ldop, stop)) logT = op.logt;   // tuned
-        if (lean_available(logR, logT, ci, co, ldop, stop)) {
+        // the repacking first pass of DCT-3 / DST-3 and invrealdft pairs lines of
+        // one transform in its tile: no more lines per tile than per transform
+        const bool mirror_in = ci && (ldop == LD_IR || ldop == LD_T3);
+        if (lean_available(logR, logT, ci, co, ldop, stop) && !(mirror_in && logL < logT + 4)) {
             a.logJ = logT + 4 - logR;
             long long nt = (a.nlines + (1ll << a.logJ) - 1) >> a.logJ;
             return launch_lean(a, logT, ci, co, ldop, stop, nt, s);
@@ -545,8 +548,10 @@ static bool run_pow2_axis(notorious_fft_plan* p, const DeviceCtx* c, const AxisP
     // otherwise an unpack epilogue reads the packed spectrum back
     bool mirror = false;
     if (op.paired && np >= 2 && !strided && !lean_disabled()) {
-        const int lr = sch.plog[np - 1];
-        mirror = recorder() ? queue_has_lean(lr, 1, 1, LD_C, op.st)
+        // (a mirror tile's lines must not outnumber the transform's: only short
+        // axes split by a tuned schedule are below that)
+        const int lr = sch.plog[np - 1], logtile = !recorder() && (sch.logt == 9 || lr > 10) ? 13 : 12;
+        mirror = logL < logtile ? false : recorder() ? queue_has_lean(lr, 1, 1, LD_C, op.st)
                             : (lr >= 4 && lean_available(lr, (lr <= 12 && lr <= 10) ? 8 : 9, 1, 1, LD_C, op.st));
     }
     const bool paired_epilogue = op.paired && !mirror;

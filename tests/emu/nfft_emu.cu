@@ -389,12 +389,12 @@ static void emu_lean(const PassArgs& a, long long t0, long long t1) {
         const long long line0 = tile << Lt::LOGJ;
         if (line0 >= a.nlines) continue;
         for (auto& x : sm) x = mkc((T)NAN, (T)NAN);
-        const long long ns = 1ll << a.logNj, tpt = Lt::MIRROR ? (ns >> Lt::LOGJ) : 1;
-        const long long tt = Lt::MIRROR ? tile - (tile / tpt) * tpt : 0;
+        const long long ns = 1ll << a.logNj, tpt = Lt::MIRROR || Lt::MIRROR_IN ? (ns >> Lt::LOGJ) : 1;
+        const long long tt = tpt > 0 ? tile - (tile / tpt) * tpt : 0;
         for (int t = 0; t < Lt::J; ++t) {
             long long tmp[3];
             TileLines tl{&tmp[0], &tmp[1], &tmp[2]};
-            if constexpr (Lt::MIRROR) {
+            if constexpr (Lt::MIRROR || Lt::MIRROR_IN) {
                 if (tpt < 1) {
                     fprintf(stderr, "nfft_emu: mirror tile larger than the transform's lines\n");
                     abort();
@@ -413,7 +413,7 @@ static void emu_lean(const PassArgs& a, long long t0, long long t1) {
         if constexpr (Lt::PREPACK) {
             // the paired repack phase, then every thread's first-sub-stage reads
             // (a barrier in the kernel) before any sub-stage write
-            for (int t = 0; t < TH; ++t) pair_prepack_thread<Lt, T, LD>(a, tw, sm.data(), lines.data(), t);
+            for (int t = 0; t < TH; ++t) pair_prepack_thread<Lt, T, LD>(a, tw, sm.data(), lines.data(), tile, t);
             std::vector<int> fl(TH), fi(TH);
             for (int t = 0; t < TH; ++t) Lt::first_smem(a, tw, sm.data(), lines.data(), t, &regs[t * 16], fl[t], fi[t]);
             for (int t = 0; t < TH; ++t) {
