@@ -15,10 +15,7 @@
 // Bound: the FP64 pipe and the exchanges (two M-point FFTs, M >= 2n, per n
 // points of traffic), so tiles are the smallest that hold a line -- 2048 points
 // and 128 threads up to M = 2048, four (FP64) or eight (FP32) CTAs per SM to
-// overlap one tile's loads with another's arithmetic.  Internal twiddles
-// W^{mk} are products of at most two table roots (loads hit L1), as exact as
-// the general kernel's lookups to one rounding; reading every root from the
-// tables instead costs half as much again (FP64 1000 x 2000: 84 us, 56 us so).
+// overlap one tile's loads with another's arithmetic.
 // B200, general kernel -> this one: FP64 1000 x 2000 150 -> 56 us, 300 x 5001
 // 174 -> 55 us, 3000 x 500 191 -> 76 us, 230 x 7 33 -> 7 us; FP32 17 x 219837
 // 210 -> 45 us, 500 x 4000 84 -> 29 us.
@@ -27,35 +24,6 @@
 #include "nfft_lean.cuh"
 
 namespace nfft {
-
-// W_{2^logP}^q from the tables, one entry where the order allows.
-template <typename T, int LOGP>
-NFFT_HD C2<T> blue_root(const TwTables<T>* tw, uint32_t q) {
-    if constexpr (LOGP <= TW_BITS) return twiddle_small<T>(tw, q, LOGP);
-    else return twiddle<T>(tw, (uint64_t)q, LOGP);
-}
-
-// v[m] *= W_{2^(LNS + LR)}^{m k}, m < 2^LR: roots of m = 1, 2, 3 and of the
-// multiples of 4 from the tables, the rest as one product of two of them.
-template <typename T, int LR, int LNS>
-NFFT_HD void blue_twiddle(const TwTables<T>* tw, int k, C2<T>* v) {
-    constexpr int RHO = 1 << LR;
-    if constexpr (LNS > 0) {
-        C2<T> lo[4];
-#pragma unroll
-        for (int m = 1; m < (RHO < 4 ? RHO : 4); ++m) {
-            lo[m] = blue_root<T, LNS + LR>(tw, (uint32_t)(m * k));
-            v[m] = cmul(v[m], lo[m]);
-        }
-#pragma unroll
-        for (int h = 4; h < RHO; h += 4) {
-            const C2<T> w = blue_root<T, LNS + LR>(tw, (uint32_t)(h * k));
-            v[h] = cmul(v[h], w);
-#pragma unroll
-            for (int m = 1; m < 4; ++m) v[h + m] = cmul(v[h + m], cmul(w, lo[m]));
-        }
-    }
-}
 
 // Radix-16 DFT of points 0..7 with points 8..15 zero.
 template <typename T> NFFT_HD void dft16_lower(C2<T>* a) {
@@ -167,7 +135,7 @@ struct Blue {
         for (int q = 0; q < 16 / RHO; ++q) {
             int l, i;
             map<LR>(t, q, l, i);
-            blue_twiddle<T, LR, LNS>(tw, i & ((1 << LNS) - 1), v + q * RHO);
+            if constexpr (LNS > 0) mul_roots<T, LR, LNS>(tw, i & ((1 << LNS) - 1), v + q * RHO);
             dft_radix<T, RHO>(v + q * RHO);
         }
     }

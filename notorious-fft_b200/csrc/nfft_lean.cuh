@@ -70,6 +70,40 @@ NFFT_HD void powers16(C2<T> x, C2<T>* p) {
     }
 }
 
+// W_{2^LOGP}^q from the tables, one entry where the order allows.
+template <typename T, int LOGP>
+NFFT_HD C2<T> table_root(const TwTables<T>* tw, uint32_t q) {
+    if constexpr (LOGP <= TW_BITS) return twiddle_small<T>(tw, q, LOGP);
+    else return twiddle<T>(tw, (uint64_t)q, LOGP);
+}
+
+// v[m] *= W_{2^(LNS + LR)}^{m k}, m < 2^LR (the internal twiddles of a
+// sub-stage): the roots of m = 1, 2, 3 and of the multiples of 4 from the
+// tables (L1 hits), the others as one product of two of them -- one rounding
+// more than a lookup, where a tree from the first root alone has up to four.
+// Reading all of them is slower (Bluestein FP64 1000 x 2000: 84 us, 56 us so).
+// The plain passes keep the tree: their tiles are bound by L1 as much as by HBM
+// (B200, FP64 4096 x 256 both ways 20.5 us with the tree, 24.6 with these loads;
+// FP32 8192 x 2000 79 and 92; radices below 16 alone, FP64 1024 x 1024 x 16 258
+// and 266).
+template <typename T, int LR, int LNS>
+NFFT_HD void mul_roots(const TwTables<T>* tw, int k, C2<T>* v) {
+    constexpr int RHO = 1 << LR;
+    C2<T> lo[4];
+#pragma unroll
+    for (int m = 1; m < (RHO < 4 ? RHO : 4); ++m) {
+        lo[m] = table_root<T, LNS + LR>(tw, (uint32_t)(m * k));
+        v[m] = cmul(v[m], lo[m]);
+    }
+#pragma unroll
+    for (int h = 4; h < RHO; h += 4) {
+        const C2<T> w = table_root<T, LNS + LR>(tw, (uint32_t)(h * k));
+        v[h] = cmul(v[h], w);
+#pragma unroll
+        for (int m = 1; m < 4; ++m) v[h + m] = cmul(v[h + m], cmul(w, lo[m]));
+    }
+}
+
 // Per-line state held by every thread of the line.
 struct LeanLine {
     long long bin, bout, j;
@@ -124,16 +158,20 @@ struct Lean {
     static constexpr int NS = LeanSched<LOGR>::n;
     static constexpr int SMEM_ELEMS = lean_smem_elems<COLL, LOGR, LOGJ>();
     static_assert(LOGJ >= 0 && LOGJ <= 8, "tile must hold 1..256 lines");
-    // paired stores need whole lines in the tile: row tiles, or mirror tiles
-    // (column in and out) for the last pass of a multi-pass transform
-    static constexpr bool MIRROR = PAIRED && COL_IN && COL_OUT;
+    // whole lines in a column tile: a real-to-real transform along a strided
+    // axis, in one pass
+    static constexpr bool WHOLE_COL = COL_IN && COL_OUT && (LOAD == LD_T2 || LOAD == LD_T3 || LOAD == LD_T4);
+    // paired stores need whole lines in the tile: row tiles, whole-line column
+    // tiles, or mirror tiles (column in and out) for the last pass of a
+    // multi-pass transform
+    static constexpr bool MIRROR = PAIRED && COL_IN && COL_OUT && !WHOLE_COL;
     // DCT-3 / DST-3 and inverse real transforms: the input repack runs as a
     // paired phase into shared memory (pair_prepack_thread) and the first
-    // sub-stage reads its points from there.  Row tiles hold whole lines; the
-    // first pass of a multi-pass transform (column in, row out) pairs line j
+    // sub-stage reads its points from there.  Row tiles and whole-line column
+    // tiles hold whole lines; the first pass of a multi-pass transform (column in, row out) pairs line j
     // with line ns - j in the tile, like the mirror tiles of the last pass.
     static constexpr bool PREPACK = LOAD == LD_T3 || LOAD == LD_IR;
-    static constexpr bool MIRROR_IN = PREPACK && COL_IN;
+    static constexpr bool MIRROR_IN = PREPACK && COL_IN && !WHOLE_COL;
     static_assert(!(MIRROR_IN && (COL_OUT || LOGJ < 1)), "the repacking pass of multi-pass transforms writes rows");
     static_assert(!(PAIRED && (COL_IN != COL_OUT)), "paired operators need row tiles or mirror tiles");
     static_assert(!MIRROR || LOGJ >= 1, "mirror tiles pair lines");
@@ -338,23 +376,22 @@ struct Lean {
         constexpr int RHO = 1 << LR;
         constexpr int lns = lns_of<S>();
         const int k = i & ((1 << lns) - 1);
-        if (k) {
-            // W^{m k} for m < RHO from the root W^k by a product tree (depth <= 4)
-            const C2<T> w1 = (lns + LR <= TW_BITS) ? twiddle_small<T>(tw, (uint32_t)k, lns + LR)
-                                                   : twiddle<T>(tw, (uint64_t)k, lns + LR);
+        if constexpr (WHOLE_COL) {
+            mul_roots<T, LR, lns>(tw, k, v);
+        } else if (k) {
+            // W^{m k} for m < RHO from the root W^k by a product tree (depth <= 4;
+            // radix 8 as a chain of six products was slower)
+            C2<T> p[16];
+            p[1] = (lns + LR <= TW_BITS) ? twiddle_small<T>(tw, (uint32_t)k, lns + LR)
+                                         : twiddle<T>(tw, (uint64_t)k, lns + LR);
             if constexpr (RHO == 16) {
-                C2<T> p[16];
-                powers16<T>(w1, p);
-#pragma unroll
-                for (int m = 1; m < 16; ++m) v[m] = cmul(v[m], p[m]);
+                powers16<T>(p[1], p);
             } else {
-                C2<T> w = w1;
 #pragma unroll
-                for (int m = 1; m < RHO; ++m) {
-                    v[m] = cmul(v[m], w);
-                    if (m + 1 < RHO) w = cmul(w, w1);
-                }
+                for (int m = 2; m < RHO; ++m) p[m] = cmul(p[m / 2], p[m - m / 2]);
             }
+#pragma unroll
+            for (int m = 1; m < RHO; ++m) v[m] = cmul(v[m], p[m]);
         }
         dft_radix<T, RHO>(v);
     }
@@ -525,13 +562,15 @@ NFFT_HD void mirror_unpack_thread(const PassArgs& a, const TwTables<T>* tw, cons
     }
 }
 
-// Row-tile paired unpack (whole lines: realdft unpack / DCT-2 post pairs), the
-// items of thread t: item w is the bin pair k, R - k (k = w mod (R/2)) of line
-// w / (R/2), R the packed spectrum length.  With
+// Paired unpack of whole lines (realdft unpack / DCT-2 post pairs), the items of
+// thread t: an item is the bin pair k, R - k of one line, R the packed spectrum
+// length.  Row tiles: item w is pair w mod (R/2) of line w / (R/2); with
 // R/2 > THREADS a thread walks one line at a time with k stepping by THREADS
 // (twiddles times the exact ratios W_N^THREADS and e^{-i pi THREADS / 2N}, at
 // most 8 products per line); otherwise its k is the same on every line and the
-// twiddles are reused.  Bin 0 (with bins M and M/2) goes through unpack_pair.
+// twiddles are reused.  Column tiles: lines fastest, so a thread stays on one
+// line with k stepping by THREADS / J (twiddles of its first pair times a table
+// root: one product).  Bin 0 (with bins M and M/2) goes through unpack_pair.
 template <typename L, typename T, int STORE>
 NFFT_HD void paired_unpack_thread(const PassArgs& a, const TwTables<T>* tw, const C2<T>* sm, const LeanLine* lines,
                                   int t) {
@@ -539,25 +578,30 @@ NFFT_HD void paired_unpack_thread(const PassArgs& a, const TwTables<T>* tw, cons
     constexpr int LOGR = L::LOGR_;
     constexpr int HALF = LOGR == 0 ? 1 : (1 << (LOGR - 1));
     constexpr int ITEMS = L::J * HALF;
+    static_assert(!L::WHOLE_COL || L::THREADS % L::J == 0, "a thread stays on one line");
     V ws = V{}, ts = V{};
-    if constexpr (HALF > L::THREADS) {
+    if constexpr (!L::WHOLE_COL && HALF > L::THREADS) {
         ws = twiddle<T>(tw, (uint64_t)L::THREADS, a.logN);
         if constexpr (STORE == ST_T2) ts = twiddle<T>(tw, (uint64_t)L::THREADS, a.logN + 2);
     }
-    V wk = V{}, tk = V{};
-    int prevk = -1;
+    V wk = V{}, tk = V{}, w0 = V{}, t0 = V{};
+    int prevk = -1, k0 = 0;
     for (int w = t; w < ITEMS; w += L::THREADS) {
-        const int ll = w / HALF, k = w & (HALF - 1);
+        const int ll = L::WHOLE_COL ? w & (L::J - 1) : w / HALF, k = L::WHOLE_COL ? w / L::J : w & (HALF - 1);
         const LeanLine ln = lines[ll];
         if (ln.j < 0) continue;
-        auto zget = [&](long long r) { return sm[NFFT_SM((lean_idx<false, LOGR, L::LOGJ>(ll, (int)r)))]; };
+        auto zget = [&](long long r) { return sm[NFFT_SM((lean_idx<L::COLL, LOGR, L::LOGJ>(ll, (int)r)))]; };
         if (k == 0) {
             unpack_pair<T, STORE>(a, tw, ln.bout, 0, (long long)(1 << LOGR), zget);
             continue;
         }
         if (prevk < 0 || k < prevk) {
-            wk = twiddle<T>(tw, (uint64_t)k, a.logN);
-            if constexpr (STORE == ST_T2) tk = twiddle<T>(tw, (uint64_t)k, a.logN + 2);
+            wk = w0 = twiddle<T>(tw, (uint64_t)k, a.logN);
+            if constexpr (STORE == ST_T2) tk = t0 = twiddle<T>(tw, (uint64_t)k, a.logN + 2);
+            k0 = k;
+        } else if constexpr (L::WHOLE_COL) {
+            wk = cmul(w0, twiddle<T>(tw, (uint64_t)(k - k0), a.logN));
+            if constexpr (STORE == ST_T2) tk = cmul(t0, twiddle<T>(tw, (uint64_t)(k - k0), a.logN + 2));
         } else if (k != prevk) {
             wk = cmul(wk, ws);
             if constexpr (STORE == ST_T2) tk = cmul(tk, ts);
@@ -578,7 +622,8 @@ NFFT_HD void paired_unpack_thread(const PassArgs& a, const TwTables<T>* tw, cons
 // a pair for each point.  Every thread has 8 items; all their loads are issued
 // before any is used, and their twiddles are one table root each times exact
 // roots of order <= 4096, so an item costs one product more than a lookup.
-// Row tiles: items walk k along a line.  Mirror-in tiles: item (l, r) is bin
+// Row tiles: items walk k along a line; whole-line column tiles: lines fastest, k
+// of a thread's line stepping by THREADS / J.  Mirror-in tiles: item (l, r) is bin
 // j + r ns of the low line j and its partner, point R - 1 - r of line ns - j;
 // the first low line of a transform's first tile (j = 0) and its high line
 // (j = ns / 2) pair with themselves (mirror_item_k).  Items walk lines fastest.
@@ -591,7 +636,7 @@ NFFT_HD void pair_prepack_thread(const PassArgs& a, const TwTables<T>* tw, C2<T>
                                  long long tile, int t) {
     using V = C2<T>;
     constexpr int LOGR = L::LOGR_, R = 1 << LOGR, NI = 8;
-    constexpr bool MIR = L::MIRROR_IN;
+    constexpr bool MIR = L::MIRROR_IN, WC = L::WHOLE_COL;
     constexpr int H = MIR ? L::J / 2 : R / 2;   // low lines of a tile / items of a line
     static_assert(MIR ? H * R == NI * L::THREADS : L::J * H == NI * L::THREADS, "8 items per thread");
     const long long es = a.in_estride;
@@ -617,7 +662,9 @@ NFFT_HD void pair_prepack_thread(const PassArgs& a, const TwTables<T>* tw, C2<T>
             lA = lB = H; rA = r - R / 2; rB = R - 1 - rA;
             return ns / 2 + rA * ns;
         } else {
-            lA = lB = w / H; rA = w & (H - 1); rB = R - rA;
+            lA = lB = WC ? w & (L::J - 1) : w / H;
+            rA = WC ? w / L::J : w & (H - 1);
+            rB = R - rA;
             return rA;
         }
     };
@@ -655,9 +702,11 @@ NFFT_HD void pair_prepack_thread(const PassArgs& a, const TwTables<T>* tw, C2<T>
         else u[q] = v[q] = mkc((T)0, (T)0);
     }
     if (half) raw(lines[MIR ? 0 : t].bin, M / 2, uh, vh);
-    // twiddles: bins of a thread step by 1 (row tiles, within a line) or D ns
+    // twiddles: bins of a thread step by THREADS (row tiles, within a line), D
+    // (column tiles) or D ns (mirror-in tiles)
     V w0 = V{}, t0 = V{};
-    constexpr int D = MIR ? L::THREADS / H : 1;
+    constexpr int D = MIR ? L::THREADS / H : WC ? L::THREADS / L::J : 1;
+    static_assert(D > 0, "a thread stays on one line");
     {
         int lA, rA, lB, rB;
         const long long k0 = item(0, lA, rA, lB, rB);
@@ -674,6 +723,11 @@ NFFT_HD void pair_prepack_thread(const PassArgs& a, const TwTables<T>* tw, C2<T>
                 wk = twiddle<T>(tw, (uint64_t)k, a.logN);
                 if constexpr (LOAD == LD_T3) tk = twiddle<T>(tw, (uint64_t)k, a.logN + 2);
             } else if (q > 0) {   // W_N^{q D ns} = W_{2R}^{q D}, e^{-i pi q D ns / 2N} = W_{8R}^{q D}
+                wk = cmul(w0, twiddle<T>(tw, (uint64_t)(q * D), LOGR + 1));
+                if constexpr (LOAD == LD_T3) tk = cmul(t0, twiddle<T>(tw, (uint64_t)(q * D), LOGR + 3));
+            }
+        } else if constexpr (WC) {   // k = k0 + q D
+            if (q > 0) {
                 wk = cmul(w0, twiddle<T>(tw, (uint64_t)(q * D), LOGR + 1));
                 if constexpr (LOAD == LD_T3) tk = cmul(t0, twiddle<T>(tw, (uint64_t)(q * D), LOGR + 3));
             }

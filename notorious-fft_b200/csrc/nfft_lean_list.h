@@ -64,6 +64,14 @@
     X(7, 8, 1, 1, LD_C, ST_BLUE) X(8, 8, 1, 1, LD_C, ST_BLUE) X(9, 8, 1, 1, LD_C, ST_BLUE)         \
     X(10, 8, 1, 1, LD_C, ST_BLUE) X(11, 9, 1, 1, LD_C, ST_BLUE)
 
+// real-to-real transforms along a strided axis (whole lines in column tiles)
+#define NFFT_LEAN_R2R_COL_ONE(X, R)                                                                \
+    X(R, 8, 1, 1, LD_T2, ST_T2) X(R, 8, 1, 1, LD_T3, ST_T3) X(R, 8, 1, 1, LD_T4, ST_T4)
+#define NFFT_LEAN_R2R_COL(X)                                                                       \
+    NFFT_LEAN_R2R_COL_ONE(X, 4) NFFT_LEAN_R2R_COL_ONE(X, 5) NFFT_LEAN_R2R_COL_ONE(X, 6)            \
+    NFFT_LEAN_R2R_COL_ONE(X, 7) NFFT_LEAN_R2R_COL_ONE(X, 8) NFFT_LEAN_R2R_COL_ONE(X, 9)            \
+    NFFT_LEAN_R2R_COL_ONE(X, 10)
+
 // the fused operators of multi-pass real and Bluestein transforms on 2048-point
 // tiles for the radices whose column tiles keep >= 8 lines (the planner takes
 // them where it prefers 128-thread tiles, as for the complex passes)
@@ -74,4 +82,4 @@
 
 #define NFFT_LEAN_ALL(X)                                                                           \
     NFFT_LEAN_C2C(X) NFFT_LEAN_REAL(X) NFFT_LEAN_MULTI(X) NFFT_LEAN_C2C_T7(X) NFFT_LEAN_BLUE(X)     \
-    NFFT_LEAN_OPS_T7(X)
+    NFFT_LEAN_R2R_COL(X) NFFT_LEAN_OPS_T7(X)

@@ -214,7 +214,11 @@ static void* get_scratch(notorious_fft_plan* p, int slot, size_t bytes) {
 
 // NOTORIOUS_FFT_GENERIC_PASSES=1 routes every pass through pass_kernel (the
 // runtime-shaped kernel), e.g. to compare it with the specialized kernels.
+// Bluestein's filter spectrum is made that way too: the general kernel's
+// twiddles are single table roots, and the filter's error is in every result.
+static thread_local bool t_general_passes = false;
 static bool lean_disabled() {
+    if (t_general_passes) return true;
     static int v = -1;
     if (v < 0) {
         const char* e = getenv("NOTORIOUS_FFT_GENERIC_PASSES");
@@ -480,7 +484,7 @@ bool run_pass(const DeviceCtx* c, const View& src, const View& dst, int logL, in
         if (op.logt && lean_available(logR, op.logt, ci, co, ldop, stop)) logT = op.logt;   // tuned
         // the repacking first pass of DCT-3 / DST-3 and invrealdft pairs lines of
         // one transform in its tile: no more lines per tile than per transform
-        const bool mirror_in = ci && (ldop == LD_IR || ldop == LD_T3);
+        const bool mirror_in = ci && !co && (ldop == LD_IR || ldop == LD_T3);
         if (lean_available(logR, logT, ci, co, ldop, stop) && !(mirror_in && logL < logT + 4)) {
             a.logJ = logT + 4 - logR;
             long long nt = (a.nlines + (1ll << a.logJ) - 1) >> a.logJ;
@@ -529,7 +533,14 @@ static bool run_pow2_axis(notorious_fft_plan* p, const DeviceCtx* c, const AxisP
     const FftSchedule& sch = strided ? ax.fft_strided : ax.fft_contig;
     const long long L = 1ll << logL;
     const int np = sch.npass;
-    if (np == 1 && !(op.paired && strided)) {
+    // a paired operator on a strided axis runs in one pass where the kernel with
+    // whole lines in column tiles exists (B200, DCT-2 + DCT-3 of 8 planes of 512 x
+    // 512 FP64 115 -> 65 us, 33 of 256 x 256 FP32 96 -> 47); otherwise through
+    // scratch and the unpack epilogue
+    const bool paired_col = op.paired && strided && np == 1 && !recorder() && !lean_disabled() && sch.plog[0] >= 4 &&
+                            src.estride != 1 && dst.estride != 1 && src.nb > 0 && src.str[0] == 1 &&
+                            lean_available(sch.plog[0], 8, 1, 1, op.ld, op.st);
+    if (np == 1 && (!(op.paired && strided) || paired_col)) {
         OpSpec o1 = op;
         o1.logt = sch.logt;
         return run_pass(c, src, dst, logL, 0, sch.plog[0], sch.tile[0], sch.nsub[0], sch.sub[0], o1, true, true, 0, 0,
@@ -792,7 +803,9 @@ static bool build_axis(notorious_fft_plan* p, const DeviceCtx* c, AxisPlan& ax, 
         vd.ptr = ax.filt;
         OpSpec op;
         op.scale = 1.0 / (double)M;
+        t_general_passes = true;
         ok = run_pow2_axis(p, c, mp, vs, vd, op, 0);
+        t_general_passes = false;
     }
     ok = ok && cuda_ok(cudaDeviceSynchronize(), "Bluestein filter");
     cudaFree(bwrap);
