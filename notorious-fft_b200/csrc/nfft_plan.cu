@@ -241,6 +241,15 @@ bool queue_has_lean(int logR, int ci, int co, int ld, int st) {
     return false;
 }
 
+static bool queue_has_blue(int logM, int ld, int st) {
+    const int k = qop_blue(logM, ld, st);
+#define X(M, LD, ST) \
+    if (k == qop_blue(M, LD, ST)) return true;
+    NFFT_QUEUE_BLUE(X)
+#undef X
+    return false;
+}
+
 // Inter-pass scratch per chunk of the outermost batch dimension
 // (NOTORIOUS_FFT_SCRATCH_MB, default 2048).  B200, FP64 2^16 x 4096 dft +
 // invdft: 32 MB chunks 2179 GB/s, 128 MB 2788, 512 MB 3187, 2048 MB 3309,
@@ -429,7 +438,10 @@ bool run_pass(const DeviceCtx* c, const View& src, const View& dst, int logL, in
         }
         const int ci = a.in_row ? 0 : 1, co = a.out_row ? 0 : 1;
         RecLaunch r;
-        if (!mid && logR >= 4 && !lean_disabled() && queue_has_lean(logR, ci, co, ldop, stop)) {
+        if (mid && a.in_row && a.out_row && !lean_disabled() && queue_has_blue(logR, ldop, stop)) {
+            a.logJ = QUEUE_LOGT + 4 - logR;
+            r.op = qop_blue(logR, ldop, stop);
+        } else if (!mid && logR >= 4 && !lean_disabled() && queue_has_lean(logR, ci, co, ldop, stop)) {
             a.logJ = QUEUE_LOGT + 4 - logR;
             r.op = qop_lean(logR, ci, co, ldop, stop);
         } else {

@@ -114,13 +114,21 @@ constexpr int QUEUE_LOG_TILE = 12;
     X(LD_BLUE_R, ST_C) X(LD_BLUE_R, ST_BLUE_R) X(LD_C, ST_BLUE_R) X(LD_BLUE_T2, ST_C)               \
     X(LD_BLUE_T2, ST_BLUE_T2) X(LD_C, ST_BLUE_T2) X(LD_FILT, ST_C)
 
+// Single-tile Bluestein branches (nfft_blue.cuh): X(LOGM, LOAD, STORE).
+#define NFFT_QUEUE_BLUE_ONE(X, M) X(M, LD_BLUE, ST_BLUE) X(M, LD_BLUE_R, ST_BLUE_R) X(M, LD_BLUE_T2, ST_BLUE_T2)
+#define NFFT_QUEUE_BLUE(X)                                                                          \
+    NFFT_QUEUE_BLUE_ONE(X, 4) NFFT_QUEUE_BLUE_ONE(X, 5) NFFT_QUEUE_BLUE_ONE(X, 6)                   \
+    NFFT_QUEUE_BLUE_ONE(X, 7) NFFT_QUEUE_BLUE_ONE(X, 8) NFFT_QUEUE_BLUE_ONE(X, 9)                   \
+    NFFT_QUEUE_BLUE_ONE(X, 10) NFFT_QUEUE_BLUE_ONE(X, 11) NFFT_QUEUE_BLUE_ONE(X, 12)
+
 // Branch keys.
 constexpr int QOP_LEAN_BASE = 0x100000, QOP_GEN_BASE = 0x200000, QOP_UNPACK_BASE = 0x300000;
-constexpr int QOP_SCALAR = 0x400000;
+constexpr int QOP_SCALAR = 0x400000, QOP_BLUE_BASE = 0x500000;
 NFFT_HD constexpr int qop_lean(int logR, int ci, int co, int ld, int st) {
     return QOP_LEAN_BASE | logR | (ci << 5) | (co << 6) | (ld << 8) | (st << 12);
 }
 NFFT_HD constexpr int qop_gen(int ld, int st) { return QOP_GEN_BASE | (ld << 8) | (st << 12); }
+NFFT_HD constexpr int qop_blue(int logM, int ld, int st) { return QOP_BLUE_BASE | logM | (ld << 8) | (st << 12); }
 NFFT_HD constexpr int qop_unpack(int st) { return QOP_UNPACK_BASE | st; }
 
 // Size-1 transforms (QOP_SCALAR): tile t covers transforms [t*SCALAR_TILE, ...)

@@ -2,11 +2,12 @@
 // (nfft_queue_kernel.cu).  Each branch runs all tiles of one queue item with
 // the same tile bodies as the standalone pass kernels.  The branches are
 // separate, non-inlined device functions, instantiated in the translation
-// units nfft_queue_b0..b4.cu (compiled in parallel as relocatable device code
+// units nfft_queue_b0..b5.cu (compiled in parallel as relocatable device code
 // with the kernel's register budget) and reached through the kernel's
 // dispatcher by the device linker.
 #pragma once
 
+#include "nfft_blue.cuh"
 #include "nfft_lean.cuh"
 #include "nfft_queue.h"
 
@@ -41,6 +42,13 @@ template <typename T, int R, int CI, int CO, int LD, int ST>
 __device__ __noinline__ void qb_lean(const QDesc* d, long long tile0, int ntiles, unsigned char* smraw) {
     for (int k = 0; k < ntiles; ++k) {
         lean_tile<T, R, QUEUE_LOGT, CI != 0, CO != 0, LD, ST>(d->a, tile0 + k, smraw);
+        __syncthreads();
+    }
+}
+template <typename T, int LOGM, int LD, int ST>
+__device__ __noinline__ void qb_blue(const QDesc* d, long long tile0, int ntiles, unsigned char* smraw) {
+    for (int k = 0; k < ntiles; ++k) {
+        blue_tile<T, LOGM, QUEUE_LOGT, LD, ST>(d->a, tile0 + k, smraw);
         __syncthreads();
     }
 }

@@ -89,13 +89,9 @@ struct BucketPlan {
 // Build options (defaults from the environment, see batch_default_options).
 struct BatchOptions {
     int use_tuned = 1;           // take pass splits from the tune cache
-    // Tiles per item.  Every item is one call of a branch function (a register
-    // save / restore of ~350 bytes per thread), so longer runs of tiles amortize
-    // it: on B200 the 20,000-transform uneven batch (FP64) took 20.65 ms at 4 / 8,
-    // 19.30 at 8 / 8, 18.76 at 16 / 16, 19.08 at 16 / 64, 19.04 at 24 / 24; the
-    // 2,000-transform batch 2.48 / 2.45 / 2.99 ms at 4 / 8, 16 / 16, 24 / 24.
-    int tiles_multi = 16;        // tiles per item of multi-pass transforms
-    int tiles_single = 16;       // tiles per item of single-pass transforms
+    // Most tiles per item (see item_tiles).
+    int tiles_multi = 16;        // multi-pass transforms
+    int tiles_single = 16;       // single-pass transforms
     long long group_bytes = 4ll << 20;
     long long lag = -1;          // items between dependent passes (-1: 3 x resident CTAs)
     long long spin_limit = 1ll << 22;
@@ -193,24 +189,43 @@ void tile_range(const RecLaunch& r, long long count, long long t0, long long t1,
     b = (t1 * lpt + J - 1) / J;
 }
 
+// A pass of one dependency group: tiles [a, b) of a descriptor.
+struct Stage {
+    int op, desc;
+    long long a, b;
+    int wait, target, done;
+};
 struct Chain {
-    std::vector<std::vector<QItem>> stages;
+    std::vector<Stage> stages;
     long long bytes = 0;
 };
 
-void add_items(std::vector<QItem>& out, int op, int desc, long long a, long long b, int per, int wait, int target,
-               int done) {
-    for (long long t = a; t < b; t += per) {
+void add_items(std::vector<QItem>& out, const Stage& s, int per) {
+    for (long long t = s.a; t < s.b; t += per) {
         QItem it;
-        it.op = op;
-        it.desc = desc;
+        it.op = s.op;
+        it.desc = s.desc;
         it.tile0 = t;
-        it.ntiles = (int)std::min<long long>(per, b - t);
-        it.wait = wait;
-        it.target = target;
-        it.done = done;
+        it.ntiles = (int)std::min<long long>(per, s.b - t);
+        it.wait = s.wait;
+        it.target = s.target;
+        it.done = s.done;
         out.push_back(it);
     }
+}
+
+// Tiles per item.  An item costs about 2 us besides its tiles (claim, descriptor
+// copy, wait, publication, the branch function's register save / restore), which
+// longer runs amortize; but an item's tiles run one after the other on one CTA
+// (6 .. 15 us each), so long runs leave the other CTAs idle when a batch has few
+// tiles or a pass of its longest transform waits for one.  So: 16 items per
+// resident CTA, 1 .. `most` tiles each.  B200, always 16 tiles -> this rule:
+// FP64, 61 transforms of up to 2^18 points 603 -> 143 us, 80 of up to 2^14 209 ->
+// 54, 1000 of up to 2^18 1730 -> 1290 (the last two with the single-tile Bluestein
+// branches); 20,000 transforms keep 16.
+int item_tiles(long long tiles, int grid, int most) {
+    const long long per = tiles / (16ll * std::max(1, grid));
+    return (int)std::max(1ll, std::min<long long>(most, per));
 }
 
 bool upload(void** dptr, const void* src, size_t bytes, const char* what) {
@@ -391,7 +406,6 @@ notorious_fft_batch* batch_create(int count, const int* kinds, const int* Ns, co
             G = std::max(g0, opt.group_bytes / per / g0 * g0);
             if (G > cnt) G = cnt;
         }
-        const int per_item = K > 1 ? opt.tiles_multi : opt.tiles_single;
         for (long long t0 = 0; t0 < cnt; t0 += G) {
             const long long t1 = std::min(cnt, t0 + G);
             Chain ch;
@@ -401,10 +415,8 @@ notorious_fft_batch* batch_create(int count, const int* kinds, const int* Ns, co
                 long long a, e;
                 tile_range(rec.launches[kk], cnt, t0, t1, a, e);
                 const int done = kk + 1 < K ? nctr++ : -1;
-                std::vector<QItem> st;
-                add_items(st, rec.launches[kk].op, desc0 + kk, a, e, per_item, prev_ctr, prev_tiles, done);
                 b->tiles += e - a;
-                ch.stages.push_back(std::move(st));
+                ch.stages.push_back(Stage{rec.launches[kk].op, desc0 + kk, a, e, prev_ctr, prev_tiles, done});
                 prev_ctr = done;
                 prev_tiles = (int)(e - a);
             }
@@ -417,6 +429,8 @@ notorious_fft_batch* batch_create(int count, const int* kinds, const int* Ns, co
         if (x.stages.size() != y.stages.size()) return x.stages.size() > y.stages.size();
         return x.bytes > y.bytes;
     });
+    const int per_multi = item_tiles(b->tiles, b->grid, opt.tiles_multi);
+    const int per_single = item_tiles(b->tiles, b->grid, opt.tiles_single);
     const long long lag = opt.lag >= 0 ? opt.lag : 3ll * b->grid;
     struct Pending {
         long long release, seq;
@@ -436,8 +450,7 @@ notorious_fft_batch* batch_create(int count, const int* kinds, const int* Ns, co
             ci = (int)next++;
             si = 0;
         }
-        auto& st = chains[ci].stages[si];
-        b->items.insert(b->items.end(), st.begin(), st.end());
+        add_items(b->items, chains[ci].stages[si], chains[ci].stages.size() > 1 ? per_multi : per_single);
         if (si + 1 < (int)chains[ci].stages.size())
             pend.push(Pending{(long long)b->items.size() + lag, seq++, ci, si + 1});
     }

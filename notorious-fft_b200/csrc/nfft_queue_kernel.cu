@@ -19,6 +19,7 @@
 // records the item in the status word; every CTA checks the flag between
 // items and in its own waits, so an abandoned launch drains quickly and the
 // context stays usable.
+#include "nfft_blue.cuh"
 #include "nfft_engine.h"
 #include "nfft_lean.cuh"
 #include "nfft_queue.h"
@@ -32,6 +33,10 @@ constexpr size_t queue_tile_smem() {
     if (lean_smem_bytes<T, R, QUEUE_LOGT, CI != 0, CO != 0, LD, ST>() > m)              \
         m = lean_smem_bytes<T, R, QUEUE_LOGT, CI != 0, CO != 0, LD, ST>();
     NFFT_QUEUE_LEAN(X)
+#undef X
+#define X(M, LD, ST)                                                                     \
+    if (blue_smem_bytes<T, M, QUEUE_LOGT, LD, ST>() > m) m = blue_smem_bytes<T, M, QUEUE_LOGT, LD, ST>();
+    NFFT_QUEUE_BLUE(X)
 #undef X
     return (m + 15) / 16 * 16;
 }
@@ -67,9 +72,11 @@ __device__ __noinline__ int queue_wait(const QueueArgs& q, int wait, unsigned ta
 }
 
 // Branch functions (nfft_queue_branches.cuh), compiled in the translation
-// units nfft_queue_b0..b4.cu and linked as relocatable device code.
+// units nfft_queue_b0..b5.cu and linked as relocatable device code.
 template <typename T, int R, int CI, int CO, int LD, int ST>
 __device__ void qb_lean(const QDesc* d, long long tile0, int ntiles, unsigned char* smraw);
+template <typename T, int LOGM, int LD, int ST>
+__device__ void qb_blue(const QDesc* d, long long tile0, int ntiles, unsigned char* smraw);
 template <typename T, int LD, int ST>
 __device__ void qb_gen(const QDesc* d, long long tile0, int ntiles, unsigned char* smraw);
 template <typename T, int ST>
@@ -84,6 +91,10 @@ __device__ __forceinline__ void queue_run_item(int op, const QDesc* d, long long
 #define X(R, CI, CO, LD, ST)                                                                  \
     case qop_lean(R, CI, CO, LD, ST): qb_lean<T, R, CI, CO, LD, ST>(d, tile0, ntiles, smraw); break;
         NFFT_QUEUE_LEAN(X)
+#undef X
+#define X(M, LD, ST)                                                                          \
+    case qop_blue(M, LD, ST): qb_blue<T, M, LD, ST>(d, tile0, ntiles, smraw); break;
+        NFFT_QUEUE_BLUE(X)
 #undef X
 #define X(LD, ST)                                                                             \
     case qop_gen(LD, ST): qb_gen<T, LD, ST>(d, tile0, ntiles, smraw); break;

@@ -1026,6 +1026,9 @@ bool launch_queue(const QueueArgs& q, int, cudaStream_t) {
 #define X(R, CI, CO, LD, ST) m[qop_lean(R, CI, CO, LD, ST)] = emu_lean<R, QUEUE_LOGT, CI != 0, CO != 0, LD, ST>;
         NFFT_QUEUE_LEAN(X)
 #undef X
+#define X(M, LD, ST) m[qop_blue(M, LD, ST)] = emu_blue<M, QUEUE_LOGT, LD, ST>;
+        NFFT_QUEUE_BLUE(X)
+#undef X
 #define X(LD, ST) m[qop_gen(LD, ST)] = emu_pass<QUEUE_LOG_TILE, LD, ST>;
         NFFT_QUEUE_GENERIC(X)
 #undef X

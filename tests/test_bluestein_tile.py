@@ -49,3 +49,48 @@ def test_gpu(lib_d, lib_f, oracle_d, n, batch, single):
         return t.cpu().numpy()
 
     check(lib_f if single else lib_d, oracle_d, n, batch, lambda a: torch.from_numpy(a).cuda(), get, True)
+
+
+# ---- the same tiles as branches of the ragged queue ---------------------------
+def check_queue(lib, oracle, put=lambda a: a, get=lambda a: a):
+    rng = np.random.default_rng(5)
+    ns = [5, 7, 9, 15, 17, 33, 63, 65, 127, 129, 255, 257, 511, 513, 1000, 1023, 1025, 2047]
+    kinds = [k for n in ns for k in ("dft", "invdft", "realdft", "dct2", "realdft")]
+    lens = [n for n in ns for _ in range(5)]
+    with lib.mkbatch(kinds, lens) as b:
+        x = rng.uniform(-1, 1, b.in_size).astype(lib.rdt)
+        y = put(np.zeros(b.out_size, lib.rdt))
+        b.execute(put(x), y)
+        assert b.status() == 0
+        y = get(y).astype(float)
+    xi = yo = 0
+    for kind, n in zip(kinds, lens):
+        cplx = kind in ("dft", "invdft")
+        ni, no = (2 * n, 2 * n) if cplx else (n, 2 * (n // 2 + 1) if kind == "realdft" else n)
+        v = x[xi:xi + ni].astype(float)
+        if cplx:
+            want = oracle.transform(kind, v[0::2] + 1j * v[1::2])
+        elif kind == "realdft":
+            want = oracle.transform("dft", v.astype(complex))[:n // 2 + 1]
+        else:
+            q = np.arange(n)
+            w = np.concatenate([v[0::2], v[1::2][::-1]]).astype(complex)
+            want = 2 * (np.exp(-0.5j * np.pi * q / n) * oracle.transform("dft", w)).real
+        got = y[yo:yo + no]
+        got = got[0::2] + 1j * got[1::2] if kind != "dct2" else got
+        assert rel_l2(got, want) <= (1e-6 if lib.single else 1e-13) * math.log2(n), (kind, n)
+        xi += ni + (ni & 1)
+        yo += no + (no & 1)
+
+
+@pytest.mark.parametrize("single", [False, True])
+def test_queue_emulated(emu_d, emu_f, oracle_d, single):
+    check_queue(emu_f if single else emu_d, oracle_d)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("single", [False, True])
+def test_queue_gpu(lib_d, lib_f, oracle_d, single):
+    import torch
+
+    check_queue(lib_f if single else lib_d, oracle_d, lambda a: torch.from_numpy(a).cuda(), lambda t: t.cpu().numpy())
