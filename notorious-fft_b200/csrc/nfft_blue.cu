@@ -42,9 +42,8 @@ bool launch_blue(PassArgs a, cudaStream_t s) {
     if (ntiles <= 0) return true;
     dim3 grid((unsigned)ntiles, 1, 1);
     if (ntiles > 0x7fffffffll) grid = dim3(0x7fffffffu, (unsigned)((ntiles + 0x7fffffffll - 1) / 0x7fffffffll), 1);
-    e->fn<<<grid, 1 << logT, e->smem, s>>>(a);
-    note_launch();
-    return cuda_ok(cudaGetLastError(), "Bluestein tile kernel launch");
+    void* args[] = {(void*)&a};
+    return cuda_ok(launch_dependent((const void*)e->fn, grid, 1 << logT, e->smem, args, s), "Bluestein tile kernel launch");
 }
 
 }  // namespace nfft

@@ -197,7 +197,7 @@ constexpr size_t blue_smem_bytes() {
 }
 
 // One tile (all threads of the CTA call it; uniform early exit past the last line).
-template <typename T, int LOGM, int LOGT, int LOAD, int STORE>
+template <typename T, int LOGM, int LOGT, int LOAD, int STORE, bool PDL = false>
 __device__ __forceinline__ void blue_tile(const PassArgs& a, long long tile, unsigned char* smraw) {
     using B = Blue<T, LOGM, LOGT, LOAD, STORE>;
     using V = C2<T>;
@@ -206,12 +206,16 @@ __device__ __forceinline__ void blue_tile(const PassArgs& a, long long tile, uns
     const TwTables<T>* tw = (const TwTables<T>*)a.tw;
     const int t = threadIdx.x;
     const long long line0 = tile << B::LOGJ;
-    if (line0 >= a.nlines) return;
+    if (line0 >= a.nlines) {
+        if constexpr (PDL) pdl_wait();
+        return;
+    }
     if (t < B::J) {
         long long tmp[3];
         line_setup(a, line0 + t, 0, TileLines{&tmp[0], &tmp[1], &tmp[2]});
         lines[t] = LeanLine{tmp[0], tmp[1], tmp[2]};
     }
+    if constexpr (PDL) pdl_wait();
     __syncthreads();
     V v[16];
     B::load(a, lines, t, v);
@@ -269,7 +273,8 @@ __global__ void __launch_bounds__(1 << blue_logt(LOGM), (lean_min_blocks<T, blue
 blue_kernel(const PassArgs a) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const long long tile = (long long)blockIdx.x + (long long)blockIdx.y * gridDim.x;
-    blue_tile<T, LOGM, blue_logt(LOGM), LD_BLUE, ST_BLUE>(a, tile, smraw);
+    pdl_trigger();
+    blue_tile<T, LOGM, blue_logt(LOGM), LD_BLUE, ST_BLUE, true>(a, tile, smraw);
 }
 
 }  // namespace nfft

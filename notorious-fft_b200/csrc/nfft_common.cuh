@@ -133,6 +133,26 @@ NFFT_HD void discard_l2(const void* p) {
 }
 
 // ---------------------------------------------------------------------------
+// Dependent launches.  Consecutive kernels of a stream overlap: a kernel lets
+// its successor be scheduled as soon as all its own CTAs run (pdl_trigger), and
+// a successor's CTAs do what needs no data (line offsets) before they wait for
+// the whole predecessor (pdl_wait: completed, its writes visible).  Every CTA of
+// a kernel launched that way waits before its first access to data and before
+// it exits, so completion stays transitive over the stream.  Tables that no
+// kernel of a stream writes (twiddles) may be read before the wait.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_trigger() {
+#if defined(__CUDA_ARCH__)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#endif
+}
+__device__ __forceinline__ void pdl_wait() {
+#if defined(__CUDA_ARCH__)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+#endif
+}
+
+// ---------------------------------------------------------------------------
 // Twiddle tables.  W_P^q = exp(-2 pi i q / P) for any power of two P <= 2^36
 // is assembled from three 4096-entry tables that split a 36-bit fraction of a
 // turn into 12-bit digits:  u = q * 2^(36 - log2 P),

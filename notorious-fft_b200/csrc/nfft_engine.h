@@ -207,7 +207,9 @@ bool run_pass(const DeviceCtx* c, const View& src, const View& dst, int logL, in
 // Inter-pass scratch layout with the lines of `like` and axis length L.
 View scratch_view(void* ptr, const View& like, long long L, bool strided);
 
-// Kernel launchers (nfft_kernels.cu)
+// Kernel launchers (nfft_kernels.cu).  launch_dependent: for kernels whose every
+// CTA calls pdl_wait() before it touches data; counts the launch.
+cudaError_t launch_dependent(const void* fn, dim3 grid, int threads, size_t smem, void** args, cudaStream_t s);
 bool launch_pass(const PassArgs& a, int load_op, int store_op, int log_tile, long long ntiles, cudaStream_t s);
 bool launch_unpack(const PassArgs& a, int store_op, const cplx_t* Z, long long zdist, long long nlines, cudaStream_t s);
 bool launch_tiny(const real_t* x, real_t* y, long long howmany, long long inner, long long idist, long long odist,

@@ -3,6 +3,7 @@
 // tables from FP64 sincospi; Bluestein chirp from exact k^2 mod 2n).
 #include "nfft_blue.h"
 
+#include <algorithm>
 #include <atomic>
 
 namespace nfft {
@@ -65,6 +66,35 @@ bool lean_available(int logR, int logT, int ci, int co, int ld, int st) {
     return lean_registry().find(lean_key(logR, logT, ci, co, ld, st)) != nullptr;
 }
 
+// Launch as a dependent of the stream's previous kernel (pdl_wait), so that the
+// launch and the line set-up overlap the predecessor's last CTAs.  B200, plain
+// launches -> these: FP64 4096 x 256 both ways 20.5 -> 17.5 us, 262144 x 4 both
+// ways 47 -> 36, realdft + invrealdft 32768 x 100 66 -> 55, 65536 x 1000 707 -> 678;
+// FP32 65536 x 1 12.3 -> 9.7.
+// Grids that fill between a quarter and half of the chip's CTA places keep
+// the plain launch: on an idle chip the scheduler spreads them over the SMs, but
+// beside a predecessor of that size the early CTAs take second places on some SMs
+// while others idle (FP64 DCT-2 + DCT-3 4096 x 230, 115 of 296 places: 26.6 us plain,
+// 30.7 dependent; FP32 256 x 256 x 33, 264 of 592: 47 and 63; from 320 of 592 up --
+// FP64 2048 x 64 x 5 22.5 and 18.8 -- and down from 128 of 592 they win).
+cudaError_t launch_dependent(const void* fn, dim3 grid, int threads, size_t smem, void** args, cudaStream_t s) {
+    // CTA places: the register budgets of lean_min_blocks on 148 SMs
+    const unsigned long long places = 148ull * (unsigned)std::max(1, (sizeof(real_t) == 8 ? 512 : 1024) / threads);
+    const unsigned long long ctas = (unsigned long long)grid.x * grid.y;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = ctas * 4 > places && ctas * 2 < places ? 0 : 1;
+    g_launches++;
+    return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
 bool launch_lean(const PassArgs& a, int logT, int ci, int co, int ld, int st, long long ntiles, cudaStream_t s) {
     const LeanEntry* e = lean_registry().find(lean_key(a.logR, logT, ci, co, ld, st));
     if (!e) {
@@ -76,9 +106,7 @@ bool launch_lean(const PassArgs& a, int logT, int ci, int co, int ld, int st, lo
     if (ntiles <= 0x7fffffffll) grid = dim3((unsigned)ntiles, 1, 1);
     else grid = dim3(0x7fffffffu, (unsigned)((ntiles + 0x7fffffffll - 1) / 0x7fffffffll), 1);
     void* args[] = {(void*)&a};
-    cudaError_t err = cudaLaunchKernel(e->fn, grid, dim3(e->threads, 1, 1), args, e->smem, s);
-    g_launches++;
-    return cuda_ok(err, "specialized pass kernel launch");
+    return cuda_ok(launch_dependent(e->fn, grid, e->threads, e->smem, args, s), "specialized pass kernel launch");
 }
 
 bool set_kernel_attributes() {
@@ -116,9 +144,9 @@ bool launch_pass(const PassArgs& a, int load_op, int store_op, int log_tile, lon
         long long gy = (ntiles + 0x7fffffffll - 1) / 0x7fffffffll;
         grid = dim3(0x7fffffffu, (unsigned)gy, 1);
     }
-    f<<<grid, threads, pass_smem_bytes<real_t>(log_tile), s>>>(a);
-    g_launches++;
-    return cuda_ok(cudaGetLastError(), "pass kernel launch");
+    void* args[] = {(void*)&a};
+    return cuda_ok(launch_dependent((const void*)f, grid, threads, pass_smem_bytes<real_t>(log_tile), args, s),
+                   "pass kernel launch");
 }
 
 bool launch_unpack(const PassArgs& a, int store_op, const cplx_t* Z, long long zdist, long long nlines, cudaStream_t s) {
@@ -128,10 +156,9 @@ bool launch_unpack(const PassArgs& a, int store_op, const cplx_t* Z, long long z
     long long blocks = (total + threads - 1) / threads;
     if (blocks > 148 * 32) blocks = 148 * 32;
     if (blocks < 1) blocks = 1;
-    if (store_op == ST_R) unpack_kernel<real_t, ST_R><<<(unsigned)blocks, threads, 0, s>>>(a, Z, zdist, nlines);
-    else unpack_kernel<real_t, ST_T2><<<(unsigned)blocks, threads, 0, s>>>(a, Z, zdist, nlines);
-    g_launches++;
-    return cuda_ok(cudaGetLastError(), "unpack kernel launch");
+    void* args[] = {(void*)&a, (void*)&Z, (void*)&zdist, (void*)&nlines};
+    const void* f = store_op == ST_R ? (const void*)unpack_kernel<real_t, ST_R> : (const void*)unpack_kernel<real_t, ST_T2>;
+    return cuda_ok(launch_dependent(f, dim3((unsigned)blocks, 1, 1), threads, 0, args, s), "unpack kernel launch");
 }
 
 bool launch_tiny(const real_t* x, real_t* y, long long howmany, long long inner, long long idist, long long odist,

@@ -768,7 +768,7 @@ NFFT_HD void pair_prepack_thread(const PassArgs& a, const TwTables<T>* tw, C2<T>
 
 // One tile of a specialized pass (all threads of the CTA call it; uniform
 // early exit past the last line).
-template <typename T, int LOGR, int LOGT, bool COL_IN, bool COL_OUT, int LOAD, int STORE>
+template <typename T, int LOGR, int LOGT, bool COL_IN, bool COL_OUT, int LOAD, int STORE, bool PDL = false>
 __device__ __forceinline__ void lean_tile(const PassArgs& a, long long tile, unsigned char* smraw) {
     using L = Lean<T, LOGR, LOGT, COL_IN, COL_OUT, LOAD, STORE>;
     using V = C2<T>;
@@ -777,7 +777,10 @@ __device__ __forceinline__ void lean_tile(const PassArgs& a, long long tile, uns
     const TwTables<T>* tw = (const TwTables<T>*)a.tw;
     const int t = threadIdx.x;
     const long long line0 = tile << L::LOGJ;
-    if (line0 >= a.nlines) return;
+    if (line0 >= a.nlines) {
+        if constexpr (PDL) pdl_wait();
+        return;
+    }
     if (t < L::J) {
         long long tmp[3];
         TileLines tl{&tmp[0], &tmp[1], &tmp[2]};
@@ -790,6 +793,7 @@ __device__ __forceinline__ void lean_tile(const PassArgs& a, long long tile, uns
         }
         lines[t] = LeanLine{tmp[0], tmp[1], tmp[2]};
     }
+    if constexpr (PDL) pdl_wait();
     __syncthreads();
 
     V v[16];
@@ -925,9 +929,10 @@ template <typename T, int LOGR, int LOGT, bool COL_IN, bool COL_OUT, int LOAD, i
 __global__ void __launch_bounds__(1 << LOGT, (lean_min_blocks<T, LOGT>()))
 lean_pass_kernel(const PassArgs a) {
     extern __shared__ __align__(16) unsigned char smraw[];
+    pdl_trigger();
     long long tile = (long long)blockIdx.x + (long long)blockIdx.y * gridDim.x;
     if constexpr (LOAD == LD_FILT) tile = lean_batch_inner(a, tile, Lean<T, LOGR, LOGT, COL_IN, COL_OUT, LOAD, STORE>::LOGJ);
-    lean_tile<T, LOGR, LOGT, COL_IN, COL_OUT, LOAD, STORE>(a, tile, smraw);
+    lean_tile<T, LOGR, LOGT, COL_IN, COL_OUT, LOAD, STORE, true>(a, tile, smraw);
 }
 
 }  // namespace nfft

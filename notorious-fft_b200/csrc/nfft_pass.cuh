@@ -360,14 +360,27 @@ struct TileLines {
     long long* j;    // Stockham line index along the axis, -1 past the end
 };
 
-// Decompose global line lam over the line dims.
+// Decompose global line lam over the line dims (32-bit divisions where the line
+// count allows, none for the outermost dim: a 64-bit division is ~100
+// instructions on every tile's critical path).
 NFFT_HD void line_setup(const PassArgs& a, long long lam, int l, TileLines tl) {
     long long bin = 0, bout = 0, j = 0;
     if (lam < a.nlines) {
+        const bool small = a.nlines <= 0x7fffffffll;
         long long rem = lam;
         for (int d = 0; d < a.ndims; ++d) {
-            long long c = rem % a.cnt[d];
-            rem /= a.cnt[d];
+            long long c = rem;
+            if (d + 1 < a.ndims) {
+                if (small) {
+                    const uint32_t n = (uint32_t)a.cnt[d], q = (uint32_t)rem / n;
+                    c = (uint32_t)rem - q * n;
+                    rem = q;
+                } else {
+                    const long long q = rem / a.cnt[d];
+                    c = rem - q * a.cnt[d];
+                    rem = q;
+                }
+            }
             if (d == a.jpos) {
                 j = c;
             } else {
@@ -536,7 +549,7 @@ template <typename T> constexpr size_t pass_smem_bytes(int log_tile) {
 
 // One tile of the generic pass (all threads of the CTA call it; uniform early
 // exit past the last line).
-template <typename T, int LOG_TILE, int LOAD, int STORE>
+template <typename T, int LOG_TILE, int LOAD, int STORE, bool PDL = false>
 __device__ __forceinline__ void pass_tile(const PassArgs& a, long long tile, unsigned char* smraw) {
     using V = C2<T>;
     constexpr int THREADS = (1 << LOG_TILE) / 16;
@@ -551,9 +564,13 @@ __device__ __forceinline__ void pass_tile(const PassArgs& a, long long tile, uns
     const int logE = a.logR + a.logJ;
     const int J = 1 << a.logJ, E = 1 << logE;
     const long long line0 = tile << a.logJ;
-    if (line0 >= a.nlines) return;
+    if (line0 >= a.nlines) {
+        if constexpr (PDL) pdl_wait();
+        return;
+    }
 
     for (int l = tid; l < J; l += THREADS) line_setup(a, line0 + l, l, tl);
+    if constexpr (PDL) pdl_wait();
     __syncthreads();
     {
         // all global loads of the slot set in flight before any is consumed
@@ -596,7 +613,8 @@ template <typename T, int LOG_TILE, int LOAD, int STORE>
 __global__ void __launch_bounds__((1 << LOG_TILE) / 16)
 pass_kernel(const PassArgs a) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    pass_tile<T, LOG_TILE, LOAD, STORE>(a, (long long)blockIdx.x + (long long)blockIdx.y * gridDim.x, smraw);
+    pdl_trigger();
+    pass_tile<T, LOG_TILE, LOAD, STORE, true>(a, (long long)blockIdx.x + (long long)blockIdx.y * gridDim.x, smraw);
 }
 
 // Paired-unpack epilogue for transforms whose packed spectrum needed more
@@ -638,6 +656,8 @@ __global__ void unpack_kernel(const PassArgs a, const C2<T>* Z, long long zdist,
     const long long M = a.N / 2;
     const long long per = M >= 2 ? M / 2 : 1;
     const long long total = per * nlines;
+    pdl_trigger();
+    pdl_wait();
     for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (long long)gridDim.x * blockDim.x)
         unpack_item<T, STORE>(a, tw, Z, zdist, w);
 }
