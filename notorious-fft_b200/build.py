@@ -27,7 +27,7 @@ BUILD = os.path.join(HERE, "_build")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 QUEUE_BRANCHES = [f"nfft_queue_b{k}.cu" for k in range(6)]
-SOURCES = ["nfft_blue.cu", "nfft_kernels.cu", "nfft_plan.cu", "nfft_api.cu", "nfft_noalloc.cu", "nfft_tc.cu",
+SOURCES = ["nfft_blue.cu", "nfft_cluster.cu", "nfft_kernels.cu", "nfft_plan.cu", "nfft_api.cu", "nfft_noalloc.cu", "nfft_tc.cu",
            "nfft_queue_build.cu", "nfft_queue_kernel.cu"] + QUEUE_BRANCHES + [f"nfft_lean_s{k}.cu" for k in range(8)] \
     + [f"nfft_pass_s{k}.cu" for k in range(4)]
 # The persistent queue kernel and its branch functions are relocatable device

@@ -2,6 +2,7 @@
 // unpack epilogue, the size-1 kernel, and the plan-time kernels (twiddle
 // tables from FP64 sincospi; Bluestein chirp from exact k^2 mod 2n).
 #include "nfft_blue.h"
+#include "nfft_cluster.h"
 
 #include <algorithm>
 #include <atomic>
@@ -110,7 +111,7 @@ bool launch_lean(const PassArgs& a, int logT, int ci, int co, int ld, int st, lo
 }
 
 bool set_kernel_attributes() {
-    if (!blue_set_attributes()) return false;
+    if (!blue_set_attributes() || !cluster_set_attributes()) return false;
     for (auto& kv : lean_registry().entries) {
         if (!cuda_ok(cudaFuncSetAttribute(kv.second.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kv.second.smem),
                      "cudaFuncSetAttribute(lean pass)"))

@@ -7,6 +7,7 @@
 #include <algorithm>
 
 #include "nfft_blue.h"
+#include "nfft_cluster.h"
 #include "nfft_engine.h"
 #include "nfft_queue.h"
 
@@ -494,6 +495,10 @@ bool run_pass(const DeviceCtx* c, const View& src, const View& dst, int logL, in
             (rr || 7 + 4 - logR >= log_jmin()))
             logT = 7;
         if (op.logt && lean_available(logR, op.logt, ci, co, ldop, stop)) logT = op.logt;   // tuned
+        // tiles that leave one CTA per SM: the same tile over a cluster (a tuned
+        // thread count selects the plain kernel where there is one)
+        if (ldop == LD_C && stop == ST_C && (!op.logt || logR > 13) && cluster_available(logR, ci, co))
+            return launch_cluster(a, ci, co, s);
         // the repacking first pass of DCT-3 / DST-3 and invrealdft pairs lines of
         // one transform in its tile: no more lines per tile than per transform
         const bool mirror_in = ci && !co && (ldop == LD_IR || ldop == LD_T3);
@@ -542,7 +547,11 @@ static bool run_pow2_axis(notorious_fft_plan* p, const DeviceCtx* c, const AxisP
                           const OpSpec& op, cudaStream_t s) {
     const int logL = ax.fft_contig.logL;
     const bool strided = !(src.estride == 1 && dst.estride == 1);
-    const FftSchedule& sch = strided ? ax.fft_strided : ax.fft_contig;
+    // one-pass schedules that only the cluster kernels run (build_axis) serve the
+    // plain form; everything else keeps the schedule without them
+    FftSchedule sch = strided ? ax.fft_strided : ax.fft_contig;
+    const bool plain = op.ld == LD_C && op.st == ST_C && !op.tc && !lean_disabled();
+    if (!plain && sch.npass == 1 && sch.plog[0] > (strided ? 13 - log_jmin() : 13)) sch = make_schedule(logL, strided);
     const long long L = 1ll << logL;
     const int np = sch.npass;
     // a paired operator on a strided axis runs in one pass where the kernel with
@@ -765,6 +774,18 @@ static bool build_axis(notorious_fft_plan* p, const DeviceCtx* c, AxisPlan& ax, 
         int logL = (family == FAM_DFT) ? ax.logn : std::max(0, ax.logn - 1);
         ax.fft_contig = make_schedule(logL, false, max_tile);
         ax.fft_strided = make_schedule(logL, true, max_tile);
+        if (family == FAM_DFT && max_tile == 13) {
+            // one pass instead of two where a cluster's tile holds the line (float:
+            // 2^14 contiguous, 2^11 strided): run_pow2_axis
+            auto one_pass = [&](FftSchedule& f, int ci) {
+                if (f.npass == 1 || !cluster_available(logL, ci, ci)) return;
+                f.npass = 1;
+                f.plog[0] = f.tile[0] = logL;
+                split_sub(logL, &f.nsub[0], f.sub[0]);
+            };
+            one_pass(ax.fft_contig, 0);
+            one_pass(ax.fft_strided, 1);
+        }
         // standalone plans: an autotuner trial, else the tune cache's split and
         // thread count for (family, n) on this GPU (a split this build cannot
         // run keeps the default schedule)

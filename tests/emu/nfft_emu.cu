@@ -198,6 +198,7 @@ __host__ __device__ void nfft_emu_smem_check(int idx) {
 #include "../../notorious-fft_b200/csrc/nfft_lean.cuh"
 #include "../../notorious-fft_b200/csrc/nfft_lean_list.h"
 #include "../../notorious-fft_b200/csrc/nfft_blue.cuh"
+#include "../../notorious-fft_b200/csrc/nfft_cluster.cuh"
 #include "../../notorious-fft_b200/csrc/nfft_tc.cuh"
 #include "../../notorious-fft_b200/csrc/nfft_tc_lean.cuh"
 #include "../../notorious-fft_b200/csrc/nfft_umma.cuh"
@@ -529,6 +530,82 @@ bool launch_blue(PassArgs a, cudaStream_t) {
     g_launches++;
     g_blue_launches++;
     tab[a.logR - BLUE_MIN_LOGM](a, 0, (a.nlines + (1ll << a.logJ) - 1) >> a.logJ);
+    return true;
+}
+
+// ---- cluster passes: the kernel body of nfft_cluster.cuh for the CTAs of a tile
+template <int LOGR, int LOGC, bool CI, bool CO>
+static void emu_cluster(const PassArgs& a, long long t0, long long t1) {
+    using T = real_t;
+    using V = C2<T>;
+    using K = Cluster<T, LOGR, LOGC, CI, CO>;
+    const TwTables<T>* tw = (const TwTables<T>*)a.tw;
+    constexpr int TH = K::THREADS;
+    g_smem_elems = K::SMEM_ELEMS;
+    std::vector<std::vector<V>> sm(K::C, std::vector<V>(K::SMEM_ELEMS));
+    std::vector<LeanLine> lines(K::J);
+    std::vector<V> regs((size_t)TH * 16);
+    std::vector<int> ls((size_t)TH * 16), is((size_t)TH * 16);
+    for (long long tile = t0; tile < t1; ++tile) {
+        for (auto& s : sm)
+            for (auto& x : s) x = mkc((T)NAN, (T)NAN);
+        for (int t = 0; t < K::J; ++t) {
+            long long tmp[3];
+            line_setup(a, (tile << K::LOGJ) + t, 0, TileLines{&tmp[0], &tmp[1], &tmp[2]});
+            lines[t] = LeanLine{tmp[0], tmp[1], tmp[2]};
+        }
+        for (int c = 0; c < K::C; ++c)
+            for (int t = 0; t < TH; ++t) {
+                int l, i;
+                V v[16];
+                K::load(a, tw, lines.data(), c, t, v, l, i);
+                for (int m = 0; m < 16; ++m) sm[m >> K::LOGM][K::at(K::sub_of(l, m), i)] = v[m];
+            }
+        for (int c = 0; c < K::C; ++c) {
+            V* s = sm[c].data();
+            for (int t = 0; t < TH; ++t) K::first(s, t, &regs[t * 16], ls[t], is[t]);
+            for (int t = 0; t < TH; ++t) K::template write<0>(s, ls[t], is[t], &regs[t * 16]);
+            auto reads = [&](auto Sc, auto Lc) {
+                constexpr int S = decltype(Sc)::value, RHO = 1 << LeanSched<LOGR - 4>::lr[S];
+                for (int t = 0; t < TH; ++t)
+                    for (int q = 0; q < 16 / RHO; ++q) {
+                        V* v = &regs[t * 16 + q * RHO];
+                        K::template read<S, decltype(Lc)::value>(s, t, q, v, ls[t * 16 + q], is[t * 16 + q]);
+                        K::Sub::template twiddle_dft<S>(tw, is[t * 16 + q], v);
+                    }
+            };
+            auto each = [&](auto Sc, auto f) {
+                constexpr int S = decltype(Sc)::value, RHO = 1 << LeanSched<LOGR - 4>::lr[S];
+                for (int t = 0; t < TH; ++t)
+                    for (int q = 0; q < 16 / RHO; ++q) f(ls[t * 16 + q], is[t * 16 + q], &regs[t * 16 + q * RHO]);
+            };
+            if constexpr (K::NS >= 3) {
+                reads(std::integral_constant<int, 1>{}, std::integral_constant<bool, K::COLL>{});
+                each(std::integral_constant<int, 1>{}, [&](int sl, int i, V* v) { K::template write<1>(s, sl, i, v); });
+            }
+            using Last = std::integral_constant<int, K::NS - 1>;
+            reads(Last{}, std::true_type{});
+            each(Last{}, [&](int sl, int i, V* v) { K::template store<Last::value>(a, lines.data(), c, sl, i, v); });
+        }
+    }
+}
+
+bool cluster_available(int logR, int ci, int co) {
+    return (ci && co) ? logR == 10 || logR == 11 : (!ci && !co && logR == CLUSTER_ROW);
+}
+static long long g_cluster_launches = 0;
+bool launch_cluster(PassArgs a, int ci, int co, cudaStream_t) {
+    if (!cluster_available(a.logR, ci, co)) {
+        set_error(6, "no cluster pass kernel for radix 2^%d", a.logR);
+        return false;
+    }
+    g_launches++;
+    g_cluster_launches++;
+    a.logJ = (sizeof(real_t) == 8 ? 13 : 14) - a.logR;
+    const long long nt = (a.nlines + (1ll << a.logJ) - 1) >> a.logJ;
+    if (!ci) emu_cluster<CLUSTER_ROW, 1, false, false>(a, 0, nt);
+    else if (a.logR == 10) emu_cluster<10, 1, true, true>(a, 0, nt);
+    else emu_cluster<11, 1, true, true>(a, 0, nt);
     return true;
 }
 
@@ -1101,6 +1178,7 @@ void nfft_emu_unregister_host(void* p) {
 }
 long long nfft_emu_launches(void) { return nfft::g_launches; }
 long long nfft_emu_lean_launches(void) { return nfft::g_lean_launches; }
+long long nfft_emu_cluster_launches(void) { return nfft::g_cluster_launches; }
 long long nfft_emu_blue_launches(void) { return nfft::g_blue_launches; }
 long long nfft_emu_checks(void) { return emu::n_checks; }
 long long nfft_emu_queue_items(void) { return nfft::g_queue_items; }
