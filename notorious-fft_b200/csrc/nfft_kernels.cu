@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <unordered_map>
 
 namespace nfft {
 
@@ -63,8 +64,16 @@ const LeanRegistry& lean_registry() {
     return reg;
 }
 
+// The registry's entries by key (every pass looks up a few of ~300).
+static const LeanEntry* lean_find(int logR, int logT, int ci, int co, int ld, int st) {
+    static const std::unordered_map<unsigned, LeanEntry> map(lean_registry().entries.begin(),
+                                                             lean_registry().entries.end());
+    const auto it = map.find(lean_key(logR, logT, ci, co, ld, st));
+    return it == map.end() ? nullptr : &it->second;
+}
+
 bool lean_available(int logR, int logT, int ci, int co, int ld, int st) {
-    return lean_registry().find(lean_key(logR, logT, ci, co, ld, st)) != nullptr;
+    return lean_find(logR, logT, ci, co, ld, st) != nullptr;
 }
 
 // Launch as a dependent of the stream's previous kernel (pdl_wait), so that the
@@ -97,7 +106,7 @@ cudaError_t launch_dependent(const void* fn, dim3 grid, int threads, size_t smem
 }
 
 bool launch_lean(const PassArgs& a, int logT, int ci, int co, int ld, int st, long long ntiles, cudaStream_t s) {
-    const LeanEntry* e = lean_registry().find(lean_key(a.logR, logT, ci, co, ld, st));
+    const LeanEntry* e = lean_find(a.logR, logT, ci, co, ld, st);
     if (!e) {
         set_error(6, "no specialized pass kernel for radix 2^%d", a.logR);
         return false;

@@ -116,6 +116,10 @@ class Library:
         L.notorious_fft_tune_lookup_plan.restype = I
         L.notorious_fft_aux_schedule.argtypes = [V, I, PI, I, PI]
         L.notorious_fft_aux_schedule.restype = I
+        self._fns = {k: getattr(L, f"notorious_fft_{k}") for k in KINDS}
+        self._fns_batched = {k: getattr(L, f"notorious_fft_{k}_batched") for k in KINDS}
+        self._fns_vjp = {k: getattr(L, f"notorious_fft_{k}_vjp") for k in KINDS}
+        self._last_error = L.notorious_fft_last_error
         self.real_size = L.notorious_fft_real_size()
         self.single = self.real_size == 4
         self.rdt = np.float32 if self.single else np.float64
@@ -132,8 +136,8 @@ class Library:
         return self.lib.notorious_fft_last_error(), self.lib.notorious_fft_last_error_string().decode()
 
     def check(self):
-        code, msg = self.last_error()
-        if code:
+        if self._last_error():
+            code, msg = self.last_error()
             raise NotoriousFFTError(f"notorious_fft error {code}: {msg}")
 
     # -- plans ------------------------------------------------------------------
@@ -196,21 +200,24 @@ class Library:
 
     # -- calls ------------------------------------------------------------------
     def _ptr(self, a):
-        if a is None:
-            return None
-        if isinstance(a, int):
+        data_ptr = getattr(a, "data_ptr", None)
+        if data_ptr is not None:
+            return data_ptr()
+        if a is None or isinstance(a, int):
             return a
-        if _is_torch(a):
-            return a.data_ptr()
         return a.ctypes.data
 
     def _call(self, fn, x, y, aux, *extra, regs=()):
+        if self._register is None:
+            fn(self._ptr(x), self._ptr(y), aux.ptr, *extra)
+            if self._last_error():
+                self.check()
+            return
         hooks = []
-        if self._register is not None:
-            for a in (x, y):
-                if isinstance(a, np.ndarray):
-                    self._register(a.ctypes.data, a.nbytes)
-                    hooks.append(a.ctypes.data)
+        for a in (x, y):
+            if isinstance(a, np.ndarray):
+                self._register(a.ctypes.data, a.nbytes)
+                hooks.append(a.ctypes.data)
         try:
             fn(self._ptr(x), self._ptr(y), aux.ptr, *extra)
         finally:
@@ -278,12 +285,11 @@ class Aux:
             y = np.empty(self.out_shape(kind), self._dtype(kind, "out"))
         if not _is_torch(x):
             x = np.ascontiguousarray(x, self._dtype(kind, "in"))
-        self.L._call(getattr(self.L.lib, f"notorious_fft_{kind}"), x, y, self)
+        self.L._call(self.L._fns[kind], x, y, self)
         return y
 
     def batched(self, kind: str, x, y, howmany: int, idist: int, odist: int):
-        self.L._call(getattr(self.L.lib, f"notorious_fft_{kind}_batched"), x, y, self, int(howmany), int(idist),
-                     int(odist))
+        self.L._call(self.L._fns_batched[kind], x, y, self, int(howmany), int(idist), int(odist))
         return y
 
     def vjp(self, kind: str, g, gx=None):
@@ -294,7 +300,7 @@ class Aux:
             gx = np.empty(self.in_shape(kind), self._dtype(kind, "in"))
         if not _is_torch(g):
             g = np.ascontiguousarray(g, self._dtype(kind, "out"))
-        self.L._call(getattr(self.L.lib, f"notorious_fft_{kind}_vjp"), g, gx, self)
+        self.L._call(self.L._fns_vjp[kind], g, gx, self)
         return gx
 
     def vjp_batched(self, kind: str, g, gx, howmany: int, idist: int, odist: int):

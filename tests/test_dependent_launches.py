@@ -81,3 +81,28 @@ def test_captured_chain(lib_d, lib_f, single):
             torch.cuda.synchronize()
             assert torch.equal(got, z), k
         del graph
+
+
+@pytest.mark.parametrize("single", [False, True])
+def test_alternating_streams(lib_d, lib_f, single):
+    """One aux (and its scratch) on the default stream and on two others in turn,
+    without a synchronization: every call waits for the one before."""
+    import torch
+    lib = lib_f if single else lib_d
+    n, batch = 1 << 17, 24
+    xs = [buffers(lib, "dft", n, batch) * (k + 1) for k in range(6)]
+    ys = [torch.zeros_like(x) for x in xs]
+    streams = [None, torch.cuda.Stream(), None, torch.cuda.Stream(), None]
+    with lib.mkaux("dft", [n]) as aux:
+        torch.cuda.synchronize()
+        for rep in range(4):
+            for k, (x, y) in enumerate(zip(xs, ys)):
+                lib.set_stream(streams[(k + rep) % len(streams)])
+                aux.batched("dft", x, y, batch, n, n)
+        lib.set_stream(None)
+        torch.cuda.synchronize()
+        want = torch.zeros_like(xs[0])
+        for x, y in zip(xs, ys):
+            aux.batched("dft", x, want, batch, n, n)
+            torch.cuda.synchronize()
+            assert torch.equal(y, want)
