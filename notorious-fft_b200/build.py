@@ -34,11 +34,12 @@ SOURCES = ["nfft_blue.cu", "nfft_cluster.cu", "nfft_kernels.cu", "nfft_plan.cu",
 # code (linked by nvcc -dlink), so the branch units compile in parallel.  They
 # read data that other CTAs wrote earlier in the same launch: global loads
 # must be served by L2 (-dlcm=cg).  The branches get the kernel's register
-# budget (256 threads, 2 CTAs per SM).
+# budget (256 threads; 2 CTAs per SM in double, 4 in float).
 RDC_SOURCES = ["nfft_queue_kernel.cu"] + QUEUE_BRANCHES
 _QUEUE_FLAGS = ["-rdc=true", "-Xptxas", "-dlcm=cg"]
 SOURCE_FLAGS = {"nfft_queue_kernel.cu": _QUEUE_FLAGS}
-SOURCE_FLAGS.update({b: _QUEUE_FLAGS + ["-maxrregcount=128"] for b in QUEUE_BRANCHES})
+SOURCE_FLAGS.update({b: _QUEUE_FLAGS for b in QUEUE_BRANCHES})
+BRANCH_REGS = {"d": ["-maxrregcount=128"], "f": ["-maxrregcount=64"]}
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 PRECISIONS = {
     "d": ("libnotorious_fft.so", ["-DNFFT_REAL=double"]),
@@ -125,7 +126,8 @@ def build(only: str | None = None, jobs: int = 8, verbose_ptxas: bool = False) -
         futs = {}
         for p in precs:
             for s in SOURCES:
-                futs[(p, s)] = ex.submit(compile_one, s, p, PRECISIONS[p][1] + SOURCE_FLAGS.get(s, []), verbose_ptxas)
+                futs[(p, s)] = ex.submit(compile_one, s, p, PRECISIONS[p][1] + SOURCE_FLAGS.get(s, [])
+                                         + (BRANCH_REGS[p] if s in QUEUE_BRANCHES else []), verbose_ptxas)
         objs = {k: f.result() for k, f in futs.items()}
     for p in precs:
         name = PRECISIONS[p][0]

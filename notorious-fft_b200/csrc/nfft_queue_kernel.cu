@@ -107,8 +107,11 @@ __device__ __forceinline__ void queue_run_item(int op, const QDesc* d, long long
     }
 }
 
+// Resident CTAs per SM, as for the standalone kernels of these tiles: the double
+// branches need their 128 registers, the float ones run in 64 (B200, FP32
+// batches of 625 uneven transforms 387 us at 2 CTAs, 303 at 4; of 1500, 1193 and 1089).
 template <typename T>
-__global__ void __launch_bounds__(QUEUE_THREADS, 2) queue_kernel(const QueueArgs q) {
+__global__ void __launch_bounds__(QUEUE_THREADS, sizeof(T) == 8 ? 2 : 4) queue_kernel(const QueueArgs q) {
     extern __shared__ __align__(16) unsigned char smraw[];
     QDesc* sd = (QDesc*)(smraw + QUEUE_TILE_SMEM);
     __shared__ long long s_item;
