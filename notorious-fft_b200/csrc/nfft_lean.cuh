@@ -567,10 +567,10 @@ NFFT_HD void mirror_unpack_thread(const PassArgs& a, const TwTables<T>* tw, cons
 // length.  Row tiles: item w is pair w mod (R/2) of line w / (R/2); with
 // R/2 > THREADS a thread walks one line at a time with k stepping by THREADS
 // (twiddles times the exact ratios W_N^THREADS and e^{-i pi THREADS / 2N}, at
-// most 8 products per line); otherwise its k is the same on every line and the
-// twiddles are reused.  Column tiles: lines fastest, so a thread stays on one
-// line with k stepping by THREADS / J (twiddles of its first pair times a table
-// root: one product).  Bin 0 (with bins M and M/2) goes through unpack_pair.
+// most 16 products per line; a table root per pair instead is 3% slower); otherwise
+// its k is the same on every line and the twiddles are reused.  Column tiles:
+// lines fastest, so a thread stays on one line with k stepping by THREADS / J
+// (twiddles of its first pair times a table root: one product).  Bin 0 (with bins M and M/2) goes through unpack_pair.
 template <typename L, typename T, int STORE>
 NFFT_HD void paired_unpack_thread(const PassArgs& a, const TwTables<T>* tw, const C2<T>* sm, const LeanLine* lines,
                                   int t) {
@@ -726,16 +726,16 @@ NFFT_HD void pair_prepack_thread(const PassArgs& a, const TwTables<T>* tw, C2<T>
                 wk = cmul(w0, twiddle<T>(tw, (uint64_t)(q * D), LOGR + 1));
                 if constexpr (LOAD == LD_T3) tk = cmul(t0, twiddle<T>(tw, (uint64_t)(q * D), LOGR + 3));
             }
-        } else if constexpr (WC) {   // k = k0 + q D
-            if (q > 0) {
-                wk = cmul(w0, twiddle<T>(tw, (uint64_t)(q * D), LOGR + 1));
-                if constexpr (LOAD == LD_T3) tk = cmul(t0, twiddle<T>(tw, (uint64_t)(q * D), LOGR + 3));
-            }
-        } else if constexpr (H > L::THREADS) {
-            constexpr int PER = H / L::THREADS, LT = L::LOGTILE - 4;
-            if (q % PER) {        // k = t + (q mod PER) THREADS
-                wk = cmul(w0, twiddle_small<T>(tw, (uint32_t)(q % PER), LOGR + 1 - LT));
-                if constexpr (LOAD == LD_T3) tk = cmul(t0, twiddle_small<T>(tw, (uint32_t)(q % PER), LOGR + 3 - LT));
+        } else if constexpr (WC || H > L::THREADS) {
+            // k = k0 + st: one table entry where the order allows, else a product
+            const int st = WC ? q * D : (q % (H > L::THREADS ? H / L::THREADS : 1)) * L::THREADS;
+            if (st) {
+                if constexpr (LOGR + 1 <= TW_BITS) wk = twiddle_small<T>(tw, (uint32_t)k, LOGR + 1);
+                else wk = cmul(w0, twiddle<T>(tw, (uint64_t)st, LOGR + 1));
+                if constexpr (LOAD == LD_T3) {
+                    if constexpr (LOGR + 3 <= TW_BITS) tk = twiddle_small<T>(tw, (uint32_t)k, LOGR + 3);
+                    else tk = cmul(t0, twiddle<T>(tw, (uint64_t)st, LOGR + 3));
+                }
             }
         }
         V zk = u[q], zm = v[q];

@@ -29,6 +29,16 @@
     NFFT_LEAN_REAL_ONE(X, 10, 8) NFFT_LEAN_REAL_ONE(X, 11, 8) NFFT_LEAN_REAL_ONE(X, 12, 8)         \
     NFFT_LEAN_REAL_ONE(X, 13, 9)
 
+// ... on 2048-point tiles, which the planner prefers: more CTAs per SM overlap
+// one tile's loads and repacking with another's arithmetic, and small batches
+// spread over more SMs (B200, 4096- -> 2048-point tiles: realdft + invrealdft FP64
+// 4096 x 2000 75 -> 68 us, 512 x 8192 37 -> 32, 128 x 295 12.3 -> 10.5; FP32 512 x 32768
+// 69 -> 62; DCT-4 FP64 2048 x 14876 139 -> 131; DST-2 + DST-3 64 x 649 19 -> 15)
+#define NFFT_LEAN_REAL_T7(X)                                                                       \
+    NFFT_LEAN_REAL_ONE(X, 4, 7) NFFT_LEAN_REAL_ONE(X, 5, 7) NFFT_LEAN_REAL_ONE(X, 6, 7)            \
+    NFFT_LEAN_REAL_ONE(X, 7, 7) NFFT_LEAN_REAL_ONE(X, 8, 7) NFFT_LEAN_REAL_ONE(X, 9, 7)            \
+    NFFT_LEAN_REAL_ONE(X, 10, 7) NFFT_LEAN_REAL_ONE(X, 11, 7)
+
 // first / last passes of multi-pass real transforms (the realdft / DCT-2 last
 // passes unpack in mirror tiles)
 #define NFFT_LEAN_MULTI_ONE(X, R, T)                                                               \
@@ -50,6 +60,9 @@
     X(8, 7, 1, 0, LD_C, ST_C) X(9, 7, 1, 0, LD_C, ST_C)                                            \
     X(4, 7, 1, 1, LD_C, ST_C) X(5, 7, 1, 1, LD_C, ST_C) X(6, 7, 1, 1, LD_C, ST_C)                  \
     X(7, 7, 1, 1, LD_C, ST_C) X(8, 7, 1, 1, LD_C, ST_C) X(9, 7, 1, 1, LD_C, ST_C)
+
+// float: 16 lines per tile along strided 512-point axes
+#define NFFT_LEAN_C2C_T9(X) X(9, 9, 1, 1, LD_C, ST_C)
 
 // multi-pass Bluestein: chirp premultiply (first forward pass), filter product
 // (first inverse pass), window + chirp postmultiply (last inverse pass)
@@ -82,4 +95,4 @@
 
 #define NFFT_LEAN_ALL(X)                                                                           \
     NFFT_LEAN_C2C(X) NFFT_LEAN_REAL(X) NFFT_LEAN_MULTI(X) NFFT_LEAN_C2C_T7(X) NFFT_LEAN_BLUE(X)     \
-    NFFT_LEAN_R2R_COL(X) NFFT_LEAN_OPS_T7(X)
+    NFFT_LEAN_R2R_COL(X) NFFT_LEAN_OPS_T7(X) NFFT_LEAN_REAL_T7(X) NFFT_LEAN_C2C_T9(X)

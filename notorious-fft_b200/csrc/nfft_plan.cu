@@ -495,6 +495,11 @@ bool run_pass(const DeviceCtx* c, const View& src, const View& dst, int logL, in
         if (lean_logt_pref(logL) == 7 && lean_available(logR, 7, ci, co, ldop, stop) &&
             (rr || 7 + 4 - logR >= log_jmin()))
             logT = 7;
+        // FP32 radix 2^9 along a strided axis: 16 lines (128 bytes) per tile row
+        // instead of 8; half spectra of 257 complex points per row leave no
+        // 64-byte row aligned (B200, rfft2 + adjoint 64 x 512 x 512 with its DCT-2
+        // 163 -> 156 us, 20 of 512 x 512 41 -> 39)
+        if (sizeof(real_t) == 4 && logR == 9 && src.estride != 1 && lean_available(logR, 9, ci, co, ldop, stop)) logT = 9;
         if (op.logt && lean_available(logR, op.logt, ci, co, ldop, stop)) logT = op.logt;   // tuned
         // tiles that leave one CTA per SM: the same tile over a cluster (a tuned
         // thread count selects the plain kernel where there is one)
