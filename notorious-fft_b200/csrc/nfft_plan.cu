@@ -557,7 +557,12 @@ static bool run_pow2_axis(notorious_fft_plan* p, const DeviceCtx* c, const AxisP
     // plain form; everything else keeps the schedule without them
     FftSchedule sch = strided ? ax.fft_strided : ax.fft_contig;
     const bool plain = op.ld == LD_C && op.st == ST_C && !op.tc && !lean_disabled();
-    if (!plain && sch.npass == 1 && sch.plog[0] > (strided ? 13 - log_jmin() : 13)) sch = make_schedule(logL, strided);
+    // (contiguous ones up to 2^25 points: a bigger batch streams faster in two plain
+    // passes.  B200, float 2^14, plain launches of two passes -> one sweep: 1001 lines
+    // 98 -> 90 us, 2000 179 -> 175, 3000 259 -> 261, 4096 350 -> 365, 8192 685 -> 735)
+    const bool big = !strided && (src.lines() << logL) > (1ll << 25);
+    if ((!plain || big) && sch.npass == 1 && sch.plog[0] > (strided ? 13 - log_jmin() : 13))
+        sch = make_schedule(logL, strided);
     const long long L = 1ll << logL;
     const int np = sch.npass;
     // a paired operator on a strided axis runs in one pass where the kernel with
