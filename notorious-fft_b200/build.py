@@ -117,7 +117,8 @@ def compile_one(src: str, prec: str, extra: list[str], verbose_ptxas: bool) -> s
     return obj
 
 
-def build(only: str | None = None, jobs: int = 8, verbose_ptxas: bool = False) -> list[str]:
+def build(only: str | None = None, jobs: int = 0, verbose_ptxas: bool = False) -> list[str]:
+    jobs = jobs or min(16, os.cpu_count() or 1)
     os.makedirs(LIB, exist_ok=True)
     os.makedirs(BUILD, exist_ok=True)
     precs = [only] if only else list(PRECISIONS)
@@ -128,6 +129,11 @@ def build(only: str | None = None, jobs: int = 8, verbose_ptxas: bool = False) -
             for s in SOURCES:
                 futs[(p, s)] = ex.submit(compile_one, s, p, PRECISIONS[p][1] + SOURCE_FLAGS.get(s, [])
                                          + (BRANCH_REGS[p] if s in QUEUE_BRANCHES else []), verbose_ptxas)
+        # the first failure is reported as it comes: what has not started is dropped
+        for f in cf.as_completed(futs.values()):
+            if f.exception():
+                ex.shutdown(wait=False, cancel_futures=True)
+                raise f.exception()
         objs = {k: f.result() for k, f in futs.items()}
     for p in precs:
         name = PRECISIONS[p][0]
@@ -159,7 +165,7 @@ if __name__ == "__main__":
     ap = argparse.ArgumentParser()
     ap.add_argument("--only", choices=sorted(PRECISIONS))
     ap.add_argument("--ptxas", action="store_true", help="print -Xptxas -v resource usage")
-    ap.add_argument("-j", type=int, default=8)
+    ap.add_argument("-j", type=int, default=0, help="files compiled at once (default: a CPU each, at most 16)")
     args = ap.parse_args()
     for o in build(args.only, args.j, args.ptxas):
         print(o)

@@ -26,11 +26,47 @@
 // scatters single points (a column layout for them) do too (FP32 16384 x 1001 127).
 #pragma once
 
-#include <cooperative_groups.h>
-
 #include "nfft_lean.cuh"
 
 namespace nfft {
+
+// Cluster primitives.  A barrier's arrive releases and its wait acquires memory at
+// cluster scope; cluster_addr is the address of this CTA's shared object p in CTA
+// `rank`'s shared memory.
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r = 0;
+#if defined(__CUDA_ARCH__)
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+#endif
+    return r;
+}
+__device__ __forceinline__ void cluster_arrive() {
+#if defined(__CUDA_ARCH__)
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+#endif
+}
+__device__ __forceinline__ void cluster_wait() {
+#if defined(__CUDA_ARCH__)
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+#endif
+}
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, unsigned rank) {
+    uint32_t r = 0;
+#if defined(__CUDA_ARCH__)
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+#endif
+    return r;
+}
+__device__ __forceinline__ void cluster_store(uint32_t addr, double2 v) {
+#if defined(__CUDA_ARCH__)
+    asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(addr), "d"(v.x), "d"(v.y) : "memory");
+#endif
+}
+__device__ __forceinline__ void cluster_store(uint32_t addr, float2 v) {
+#if defined(__CUDA_ARCH__)
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
+#endif
+}
 
 template <typename T, int LOGR, int LOGC, bool COL_IN, bool COL_OUT>
 struct Cluster {
@@ -153,14 +189,12 @@ template <typename T, int LOGR, int LOGC, bool COL_IN, bool COL_OUT>
 __global__ void __launch_bounds__(sizeof(T) == 8 ? 256 : 512, 2) cluster_kernel(const PassArgs a) {
     using K = Cluster<T, LOGR, LOGC, COL_IN, COL_OUT>;
     using V = C2<T>;
-    namespace cg = cooperative_groups;
     extern __shared__ __align__(16) unsigned char smraw[];
     V* sm = (V*)smraw;
     LeanLine* lines = (LeanLine*)(sm + K::SMEM_ELEMS);
     const TwTables<T>* tw = (const TwTables<T>*)a.tw;
     const int t = threadIdx.x;
-    cg::cluster_group cl = cg::this_cluster();
-    const int c = (int)cl.block_rank();
+    const int c = (int)cluster_rank();
     pdl_trigger();
     const long long tile = (long long)blockIdx.x >> LOGC;   // every CTA of the grid has a tile
     if (t < K::J) {
@@ -168,19 +202,18 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 256 : 512, 2) cluster_kernel(
         line_setup(a, (tile << K::LOGJ) + t, 0, TileLines{&tmp[0], &tmp[1], &tmp[2]});
         lines[t] = LeanLine{tmp[0], tmp[1], tmp[2]};
     }
-    cl.barrier_arrive();   // every CTA of the cluster runs before any writes to its memory
+    cluster_arrive();   // every CTA of the cluster runs before any writes to its memory
     pdl_wait();
     __syncthreads();
     V v[16];
     int l, i;
     K::load(a, tw, lines, c, t, v, l, i);
-    cl.barrier_wait();
+    cluster_wait();
 #pragma unroll
-    for (int m = 0; m < 16; ++m) {
-        V* to = cl.map_shared_rank(sm, m >> K::LOGM);
-        to[K::at(K::sub_of(l, m), i)] = v[m];
-    }
-    cl.sync();   // the sub-lines are complete; no writes to other CTAs after this
+    for (int m = 0; m < 16; ++m)
+        cluster_store(cluster_addr(sm, m >> K::LOGM) + (uint32_t)(sizeof(V) * K::at(K::sub_of(l, m), i)), v[m]);
+    cluster_arrive();   // the sub-lines are complete; no writes to other CTAs after this
+    cluster_wait();
     int s;
     K::first(sm, t, v, s, i);
     __syncthreads();
