@@ -379,16 +379,20 @@ struct Lean {
         if constexpr (WHOLE_COL) {
             mul_roots<T, LR, lns>(tw, k, v);
         } else if (k) {
-            // W^{m k} for m < RHO from the root W^k by a product tree (depth <= 4;
-            // radix 8 as a chain of six products was slower)
+            // W^{m k} for m < RHO from the root W^k by products (depth <= 4); radix 8
+            // takes W^{4 k} from the table too.  From W^k alone its error grows
+            // with m: as a tree it was 3% above a chain of six products in the
+            // result of a 128- or 512-point transform, as a chain slower; with the
+            // second root it is below both.
             C2<T> p[16];
-            p[1] = (lns + LR <= TW_BITS) ? twiddle_small<T>(tw, (uint32_t)k, lns + LR)
-                                         : twiddle<T>(tw, (uint64_t)k, lns + LR);
+            p[1] = table_root<T, lns + LR>(tw, (uint32_t)k);
             if constexpr (RHO == 16) {
                 powers16<T>(p[1], p);
             } else {
+                if constexpr (RHO == 8) p[4] = table_root<T, lns + LR>(tw, (uint32_t)(4 * k));
 #pragma unroll
-                for (int m = 2; m < RHO; ++m) p[m] = cmul(p[m / 2], p[m - m / 2]);
+                for (int m = 2; m < RHO; ++m)
+                    if (m != 4) p[m] = cmul(p[m & 4 ? 4 : m / 2], p[m & 4 ? m - 4 : m - m / 2]);
             }
 #pragma unroll
             for (int m = 1; m < RHO; ++m) v[m] = cmul(v[m], p[m]);
