@@ -624,8 +624,7 @@ NFFT_HD void paired_unpack_thread(const PassArgs& a, const TwTables<T>* tw, cons
 // (W_N^{M-k} = -conj W_N^k and e^{-i pi (M-k)/2N} = e^{-i pi/4} conj
 // e^{-i pi k/2N} exactly), where the generic operators compute both members of
 // a pair for each point.  Every thread has 8 items; all their loads are issued
-// before any is used, and their twiddles are one table root each times exact
-// roots of order <= 4096, so an item costs one product more than a lookup.
+// before any is used; their twiddles are the tables' roots.
 // Row tiles: items walk k along a line; whole-line column tiles: lines fastest, k
 // of a thread's line stepping by THREADS / J.  Mirror-in tiles: item (l, r) is bin
 // j + r ns of the low line j and its partner, point R - 1 - r of line ns - j;
@@ -706,41 +705,21 @@ NFFT_HD void pair_prepack_thread(const PassArgs& a, const TwTables<T>* tw, C2<T>
         else u[q] = v[q] = mkc((T)0, (T)0);
     }
     if (half) raw(lines[MIR ? 0 : t].bin, M / 2, uh, vh);
-    // twiddles: bins of a thread step by THREADS (row tiles, within a line), D
-    // (column tiles) or D ns (mirror-in tiles)
-    V w0 = V{}, t0 = V{};
-    constexpr int D = MIR ? L::THREADS / H : WC ? L::THREADS / L::J : 1;
-    static_assert(D > 0, "a thread stays on one line");
-    {
-        int lA, rA, lB, rB;
-        const long long k0 = item(0, lA, rA, lB, rB);
-        w0 = twiddle<T>(tw, (uint64_t)k0, a.logN);
-        if constexpr (LOAD == LD_T3) t0 = twiddle<T>(tw, (uint64_t)k0, a.logN + 2);
-    }
+    // Twiddles from the tables, pair by pair: as products of the thread's first root
+    // with exact ones they cost a rounding more (DCT-3 of 8192 points and more, error
+    // up to 4% larger).  Row tiles of short lines have the same k in every pair.
+    constexpr bool SAME_K = !MIR && !WC && H <= L::THREADS;
+    V wk = V{}, tk = V{};
 #pragma unroll
     for (int q = 0; q < NI; ++q) {
         int lA, rA, lB, rB;
         const long long k = item(q, lA, rA, lB, rB);
-        V wk = w0, tk = t0;
         if constexpr (MIR) {
-            if (self) {
-                wk = twiddle<T>(tw, (uint64_t)k, a.logN);
-                if constexpr (LOAD == LD_T3) tk = twiddle<T>(tw, (uint64_t)k, a.logN + 2);
-            } else if (q > 0) {   // W_N^{q D ns} = W_{2R}^{q D}, e^{-i pi q D ns / 2N} = W_{8R}^{q D}
-                wk = cmul(w0, twiddle<T>(tw, (uint64_t)(q * D), LOGR + 1));
-                if constexpr (LOAD == LD_T3) tk = cmul(t0, twiddle<T>(tw, (uint64_t)(q * D), LOGR + 3));
-            }
-        } else if constexpr (WC || H > L::THREADS) {
-            // k = k0 + st: one table entry where the order allows, else a product
-            const int st = WC ? q * D : (q % (H > L::THREADS ? H / L::THREADS : 1)) * L::THREADS;
-            if (st) {
-                if constexpr (LOGR + 1 <= TW_BITS) wk = twiddle_small<T>(tw, (uint32_t)k, LOGR + 1);
-                else wk = cmul(w0, twiddle<T>(tw, (uint64_t)st, LOGR + 1));
-                if constexpr (LOAD == LD_T3) {
-                    if constexpr (LOGR + 3 <= TW_BITS) tk = twiddle_small<T>(tw, (uint32_t)k, LOGR + 3);
-                    else tk = cmul(t0, twiddle<T>(tw, (uint64_t)st, LOGR + 3));
-                }
-            }
+            wk = twiddle<T>(tw, (uint64_t)k, a.logN);
+            if constexpr (LOAD == LD_T3) tk = twiddle<T>(tw, (uint64_t)k, a.logN + 2);
+        } else if (q == 0 || !SAME_K) {
+            wk = table_root<T, LOGR + 1>(tw, (uint32_t)k);
+            if constexpr (LOAD == LD_T3) tk = table_root<T, LOGR + 3>(tw, (uint32_t)k);
         }
         V zk = u[q], zm = v[q];
         if constexpr (LOAD == LD_IR) {

@@ -67,6 +67,11 @@ BOUNDS = [
     ("realdft", (256,), 128, 2.572e-16, 1.310e-07),
     ("dct2", (1024,), 32, 3.126e-16, 1.554e-07),
     ("dft", (512, 32), 1, 3.080e-16, 1.604e-07),
+    # input repack of DCT-3 / DST-3 and invrealdft
+    ("dct3", (8192,), 4, 5.345e-16, 3.069e-07),
+    ("dct3", (16384,), 2, 4.726e-16, 2.540e-07),
+    ("dst3", (32768,), 1, 5.211e-16, 2.823e-07),
+    ("invrealdft", (16384,), 2, 4.557e-16, 2.467e-07),
 ]
 
 
