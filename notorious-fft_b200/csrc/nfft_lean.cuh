@@ -570,9 +570,11 @@ NFFT_HD void mirror_unpack_thread(const PassArgs& a, const TwTables<T>* tw, cons
 // thread t: an item is the bin pair k, R - k of one line, R the packed spectrum
 // length.  Row tiles: item w is pair w mod (R/2) of line w / (R/2); with
 // R/2 > THREADS a thread walks one line at a time with k stepping by THREADS
-// (twiddles times the exact ratios W_N^THREADS and e^{-i pi THREADS / 2N}, at
-// most 16 products per line; a table root per pair instead is 3% slower); otherwise
-// its k is the same on every line and the twiddles are reused.  Column tiles:
+// (twiddles times the exact ratios W_N^THREADS and e^{-i pi THREADS / 2N}; a table
+// root per pair instead is 3% slower at 8192 points), taking a new root from the
+// table after R/512 pairs: the chain of a 256-thread tile, whatever the tile.
+// Otherwise its k is the same on every line and the twiddles are reused.
+// Column tiles:
 // lines fastest, so a thread stays on one line with k stepping by THREADS / J
 // (twiddles of its first pair times a table root: one product).  Bin 0 (with bins M and M/2) goes through unpack_pair.
 template <typename L, typename T, int STORE>
@@ -590,6 +592,7 @@ NFFT_HD void paired_unpack_thread(const PassArgs& a, const TwTables<T>* tw, cons
     }
     V wk = V{}, tk = V{}, w0 = V{}, t0 = V{};
     int prevk = -1, k0 = 0;
+    constexpr int CHAIN = HALF < 256 ? 1 : HALF / 256;   // pairs per table root
     for (int w = t; w < ITEMS; w += L::THREADS) {
         const int ll = L::WHOLE_COL ? w & (L::J - 1) : w / HALF, k = L::WHOLE_COL ? w / L::J : w & (HALF - 1);
         const LeanLine ln = lines[ll];
@@ -599,7 +602,7 @@ NFFT_HD void paired_unpack_thread(const PassArgs& a, const TwTables<T>* tw, cons
             unpack_pair<T, STORE>(a, tw, ln.bout, 0, (long long)(1 << LOGR), zget);
             continue;
         }
-        if (prevk < 0 || k < prevk) {
+        if (prevk < 0 || k < prevk || (!L::WHOLE_COL && k != prevk && (k / L::THREADS) % CHAIN == 0)) {
             wk = w0 = twiddle<T>(tw, (uint64_t)k, a.logN);
             if constexpr (STORE == ST_T2) tk = t0 = twiddle<T>(tw, (uint64_t)k, a.logN + 2);
             k0 = k;

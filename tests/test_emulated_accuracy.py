@@ -72,6 +72,12 @@ BOUNDS = [
     ("dct3", (16384,), 2, 4.726e-16, 2.540e-07),
     ("dst3", (32768,), 1, 5.211e-16, 2.823e-07),
     ("invrealdft", (16384,), 2, 4.557e-16, 2.467e-07),
+    # output unpack of realdft and DCT-2 / DST-2, whole lines
+    ("realdft", (2048,), 16, 3.941e-16, 2.191e-07),
+    ("realdft", (4096,), 8, 4.302e-16, 2.414e-07),
+    ("dct2", (2048,), 16, 4.083e-16, 2.339e-07),
+    ("dct2", (4096,), 8, 4.632e-16, 2.557e-07),
+    ("dst2", (4096,), 8, 4.616e-16, 2.548e-07),
 ]
 
 
