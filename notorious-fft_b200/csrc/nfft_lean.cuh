@@ -104,6 +104,14 @@ NFFT_HD void mul_roots(const TwTables<T>* tw, int k, C2<T>* v) {
     }
 }
 
+// The same with every root from the tables: for column tiles, where the lines of a
+// tile share k and a warp reads few entries at a time.
+template <typename T, int LR, int LNS>
+NFFT_HD void mul_table(const TwTables<T>* tw, int k, C2<T>* v) {
+#pragma unroll
+    for (int m = 1; m < (1 << LR); ++m) v[m] = cmul(v[m], table_root<T, LNS + LR>(tw, (uint32_t)(m * k)));
+}
+
 // Per-line state held by every thread of the line.
 struct LeanLine {
     long long bin, bout, j;
@@ -377,7 +385,7 @@ struct Lean {
         constexpr int lns = lns_of<S>();
         const int k = i & ((1 << lns) - 1);
         if constexpr (WHOLE_COL) {
-            mul_roots<T, LR, lns>(tw, k, v);
+            mul_table<T, LR, lns>(tw, k, v);
         } else if (k) {
             // W^{m k} for m < RHO from the root W^k by products (depth <= 4); radix 8
             // takes W^{4 k} from the table too.  From W^k alone its error grows
@@ -574,9 +582,8 @@ NFFT_HD void mirror_unpack_thread(const PassArgs& a, const TwTables<T>* tw, cons
 // root per pair instead is 3% slower at 8192 points), taking a new root from the
 // table after R/512 pairs: the chain of a 256-thread tile, whatever the tile.
 // Otherwise its k is the same on every line and the twiddles are reused.
-// Column tiles:
-// lines fastest, so a thread stays on one line with k stepping by THREADS / J
-// (twiddles of its first pair times a table root: one product).  Bin 0 (with bins M and M/2) goes through unpack_pair.
+// Column tiles: lines fastest, k stepping by THREADS / J, every root from the tables
+// (the lines of a tile share it).  Bin 0 (with bins M and M/2) goes through unpack_pair.
 template <typename L, typename T, int STORE>
 NFFT_HD void paired_unpack_thread(const PassArgs& a, const TwTables<T>* tw, const C2<T>* sm, const LeanLine* lines,
                                   int t) {
@@ -584,14 +591,13 @@ NFFT_HD void paired_unpack_thread(const PassArgs& a, const TwTables<T>* tw, cons
     constexpr int LOGR = L::LOGR_;
     constexpr int HALF = LOGR == 0 ? 1 : (1 << (LOGR - 1));
     constexpr int ITEMS = L::J * HALF;
-    static_assert(!L::WHOLE_COL || L::THREADS % L::J == 0, "a thread stays on one line");
     V ws = V{}, ts = V{};
     if constexpr (!L::WHOLE_COL && HALF > L::THREADS) {
         ws = twiddle<T>(tw, (uint64_t)L::THREADS, a.logN);
         if constexpr (STORE == ST_T2) ts = twiddle<T>(tw, (uint64_t)L::THREADS, a.logN + 2);
     }
-    V wk = V{}, tk = V{}, w0 = V{}, t0 = V{};
-    int prevk = -1, k0 = 0;
+    V wk = V{}, tk = V{};
+    int prevk = -1;
     constexpr int CHAIN = HALF < 256 ? 1 : HALF / 256;   // pairs per table root
     for (int w = t; w < ITEMS; w += L::THREADS) {
         const int ll = L::WHOLE_COL ? w & (L::J - 1) : w / HALF, k = L::WHOLE_COL ? w / L::J : w & (HALF - 1);
@@ -602,13 +608,9 @@ NFFT_HD void paired_unpack_thread(const PassArgs& a, const TwTables<T>* tw, cons
             unpack_pair<T, STORE>(a, tw, ln.bout, 0, (long long)(1 << LOGR), zget);
             continue;
         }
-        if (prevk < 0 || k < prevk || (!L::WHOLE_COL && k != prevk && (k / L::THREADS) % CHAIN == 0)) {
-            wk = w0 = twiddle<T>(tw, (uint64_t)k, a.logN);
-            if constexpr (STORE == ST_T2) tk = t0 = twiddle<T>(tw, (uint64_t)k, a.logN + 2);
-            k0 = k;
-        } else if constexpr (L::WHOLE_COL) {
-            wk = cmul(w0, twiddle<T>(tw, (uint64_t)(k - k0), a.logN));
-            if constexpr (STORE == ST_T2) tk = cmul(t0, twiddle<T>(tw, (uint64_t)(k - k0), a.logN + 2));
+        if (L::WHOLE_COL || prevk < 0 || k < prevk || (k != prevk && (k / L::THREADS) % CHAIN == 0)) {
+            wk = twiddle<T>(tw, (uint64_t)k, a.logN);
+            if constexpr (STORE == ST_T2) tk = twiddle<T>(tw, (uint64_t)k, a.logN + 2);
         } else if (k != prevk) {
             wk = cmul(wk, ws);
             if constexpr (STORE == ST_T2) tk = cmul(tk, ts);
@@ -624,9 +626,9 @@ NFFT_HD void paired_unpack_thread(const PassArgs& a, const TwTables<T>* tw, cons
 // realdft) and DCT-3 / DST-3 (z = the pre-twiddled reorder zb of the reals;
 // zb_0 doubled for the adjoint of DCT-2 / DST-2).  An item is a pair of bins k,
 // M - k: it takes z_k and z_{M-k} once and writes both points
-// (W_N^{M-k} = -conj W_N^k and e^{-i pi (M-k)/2N} = e^{-i pi/4} conj
-// e^{-i pi k/2N} exactly), where the generic operators compute both members of
-// a pair for each point.  Every thread has 8 items; all their loads are issued
+// (W_N^{M-k} = -conj W_N^k; in row tiles e^{-i pi (M-k)/2N} = e^{-i pi/4} conj
+// e^{-i pi k/2N}, one lookup less for two roundings more), where the generic
+// operators compute both members of a pair for each point.  Every thread has 8 items; all their loads are issued
 // before any is used; their twiddles are the tables' roots.
 // Row tiles: items walk k along a line; whole-line column tiles: lines fastest, k
 // of a thread's line stepping by THREADS / J.  Mirror-in tiles: item (l, r) is bin
@@ -712,17 +714,24 @@ NFFT_HD void pair_prepack_thread(const PassArgs& a, const TwTables<T>* tw, C2<T>
     // with exact ones they cost a rounding more (DCT-3 of 8192 points and more, error
     // up to 4% larger).  Row tiles of short lines have the same k in every pair.
     constexpr bool SAME_K = !MIR && !WC && H <= L::THREADS;
-    V wk = V{}, tk = V{};
+    V wk = V{}, tk = V{}, tm = V{};
 #pragma unroll
     for (int q = 0; q < NI; ++q) {
         int lA, rA, lB, rB;
         const long long k = item(q, lA, rA, lB, rB);
         if constexpr (MIR) {
             wk = twiddle<T>(tw, (uint64_t)k, a.logN);
-            if constexpr (LOAD == LD_T3) tk = twiddle<T>(tw, (uint64_t)k, a.logN + 2);
+            if constexpr (LOAD == LD_T3) {
+                tk = twiddle<T>(tw, (uint64_t)k, a.logN + 2);
+                tm = twiddle<T>(tw, (uint64_t)(M - k), a.logN + 2);
+            }
         } else if (q == 0 || !SAME_K) {
             wk = table_root<T, LOGR + 1>(tw, (uint32_t)k);
-            if constexpr (LOAD == LD_T3) tk = table_root<T, LOGR + 3>(tw, (uint32_t)k);
+            if constexpr (LOAD == LD_T3) {
+                tk = table_root<T, LOGR + 3>(tw, (uint32_t)k);
+                if constexpr (WC) tm = table_root<T, LOGR + 3>(tw, (uint32_t)(M - k));
+                else tm = mkc((tk.x - tk.y) * K<T>::r2, -(tk.x + tk.y) * K<T>::r2);
+            }
         }
         V zk = u[q], zm = v[q];
         if constexpr (LOAD == LD_IR) {
@@ -733,7 +742,7 @@ NFFT_HD void pair_prepack_thread(const PassArgs& a, const TwTables<T>* tw, C2<T>
         } else {
             if (k == 0) zk = mkc(a.vjp ? (T)2 * zk.x : zk.x, (T)0);
             else zk = pre(zk, tk);
-            zm = pre(zm, mkc((tk.x - tk.y) * K<T>::r2, -(tk.x + tk.y) * K<T>::r2));
+            zm = pre(zm, tm);
         }
         if (k == 0) {
             put(lA, 0, mkc(zk.x + zm.x, zm.x - zk.x));

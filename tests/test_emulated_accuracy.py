@@ -78,6 +78,14 @@ BOUNDS = [
     ("dct2", (2048,), 16, 4.083e-16, 2.339e-07),
     ("dct2", (4096,), 8, 4.632e-16, 2.557e-07),
     ("dst2", (4096,), 8, 4.616e-16, 2.548e-07),
+    # real-to-real transforms along strided axes; second twiddle of the multi-pass repack
+    ("dct2", (64, 32), 8, 2.610e-16, 1.455e-07),
+    ("dst2", (32, 32), 8, 2.529e-16, 1.422e-07),
+    ("dct3", (256, 32), 4, 2.814e-16, 1.513e-07),
+    ("dct3", (2048, 32), 1, 3.047e-16, 1.682e-07),
+    ("dst3", (512, 32), 2, 2.863e-16, 1.577e-07),
+    ("dct4", (1024, 32), 1, 5.721e-16, 1.578e-07),
+    ("dct3", (131072,), 1, 6.411e-16, 3.640e-07),
 ]
 
 
