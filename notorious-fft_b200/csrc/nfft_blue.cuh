@@ -135,7 +135,9 @@ struct Blue {
         for (int q = 0; q < 16 / RHO; ++q) {
             int l, i;
             map<LR>(t, q, l, i);
-            if constexpr (LNS > 0) mul_roots<T, LR, LNS>(tw, i & ((1 << LNS) - 1), v + q * RHO);
+            // up to 8 different k: few entries per load, so all roots come from the tables
+            if constexpr (LNS > 3) mul_roots<T, LR, LNS>(tw, i & ((1 << LNS) - 1), v + q * RHO);
+            else if constexpr (LNS > 0) mul_table<T, LR, LNS>(tw, i & ((1 << LNS) - 1), v + q * RHO);
             dft_radix<T, RHO>(v + q * RHO);
         }
     }

@@ -215,9 +215,9 @@ static void* get_scratch(notorious_fft_plan* p, int slot, size_t bytes) {
 
 // NOTORIOUS_FFT_GENERIC_PASSES=1 routes every pass through pass_kernel (the
 // runtime-shaped kernel), e.g. to compare it with the specialized kernels.
-// Bluestein's filter spectrum of single-tile lengths is made that way too: the
-// general kernel's twiddles are single table roots, and the filter's error is in
-// every result (longer filters would make a plan 30 us dearer).
+// Bluestein's filter spectrum of single-tile lengths (padded up to 2^13) is made that
+// way too: the general kernel's twiddles are single table roots, and the filter's
+// error is in every result.
 static thread_local bool t_general_passes = false;
 static bool lean_disabled() {
     if (t_general_passes) return true;
@@ -847,7 +847,7 @@ static bool build_axis(notorious_fft_plan* p, const DeviceCtx* c, AxisPlan& ax, 
         vd.ptr = ax.filt;
         OpSpec op;
         op.scale = 1.0 / (double)M;
-        t_general_passes = ax.logM <= 12;
+        t_general_passes = ax.logM <= BLUE_MAX_LOGM;
         ok = run_pow2_axis(p, c, mp, vs, vd, op, 0);
         t_general_passes = false;
     }

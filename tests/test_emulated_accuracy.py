@@ -86,6 +86,12 @@ BOUNDS = [
     ("dst3", (512, 32), 2, 2.863e-16, 1.577e-07),
     ("dct4", (1024, 32), 1, 5.721e-16, 1.578e-07),
     ("dct3", (131072,), 1, 6.411e-16, 3.640e-07),
+    # Bluestein in one tile, padded to 2^13
+    ("dft", (2049,), 7, 4.317e-16, 2.458e-07),
+    ("dft", (2100,), 7, 4.386e-16, 2.510e-07),
+    ("invdft", (2500,), 6, 4.993e-16, 2.777e-07),
+    ("dft", (3000,), 5, 5.059e-16, 2.830e-07),
+    ("dft", (4095,), 4, 5.758e-16, 3.296e-07),
 ]
 
 
