@@ -254,11 +254,8 @@ bool run_pipelined(notorious_fft_plan* p, int kind, const void* x, void* y, long
 
 // Calls on one plan share its device scratch.  Calls on one stream are
 // ordered by that stream; a call on a different stream than the previous
-// call first waits for the previous call's work: an event recorded at the end
-// of the call, or, for the legacy default stream, when the other stream's call
-// comes (that stream is never destroyed, and an event between two calls would
-// keep the second one's kernels from overlapping the first one's: FP64 1024 x 1,
-// back to back through the binding, 6.1 us a call with it, 5.0 without).  Streams being captured into a CUDA graph are neither made
+// call first waits for the previous call's work (an event recorded at the end
+// of every call).  Streams being captured into a CUDA graph are neither made
 // to wait nor recorded: ordering a capture against earlier calls on other
 // streams is the caller's (synchronize before capturing).
 bool is_capturing(cudaStream_t s) {
@@ -270,31 +267,16 @@ bool is_capturing(cudaStream_t s) {
     return st != cudaStreamCaptureStatusNone;
 }
 
-bool ensure_event(notorious_fft_plan* p) {
-    return p->ev_last || cuda_ok(cudaEventCreateWithFlags(&p->ev_last, cudaEventDisableTiming), "cudaEventCreate");
-}
-
 bool order_after_previous_call(notorious_fft_plan* p, cudaStream_t s, bool capturing) {
     if (capturing || !p->ev_pending || p->last_stream == s) return true;
-    if (!p->last_stream) {
-        // legal while another thread captures a stream of its own
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-        cudaThreadExchangeStreamCaptureMode(&mode);
-        const bool ok = ensure_event(p) && cuda_ok(cudaEventRecord(p->ev_last, p->last_stream), "cudaEventRecord(call end)");
-        cudaThreadExchangeStreamCaptureMode(&mode);
-        if (!ok) return false;
-    }
     return cuda_ok(cudaStreamWaitEvent(s, p->ev_last, 0), "cudaStreamWaitEvent(previous call)");
 }
 
 void note_call(notorious_fft_plan* p, cudaStream_t s, bool capturing) {
     if (capturing) return;
-    if (!s) {   // order_after_previous_call records
-        p->last_stream = s;
-        p->ev_pending = true;
+    if (!p->ev_last && !cuda_ok(cudaEventCreateWithFlags(&p->ev_last, cudaEventDisableTiming), "cudaEventCreate"))
         return;
-    }
-    if (ensure_event(p) && cuda_ok(cudaEventRecord(p->ev_last, s), "cudaEventRecord(call end)")) {
+    if (cuda_ok(cudaEventRecord(p->ev_last, s), "cudaEventRecord(call end)")) {
         p->last_stream = s;
         p->ev_pending = true;
     }

@@ -190,7 +190,6 @@ __host__ __device__ void nfft_emu_smem_check(int idx) {
 #define cudaStreamWaitEvent(s, e, f) emu::Ok()
 #define cudaEventDestroy(e) emu::Ok()
 #define cudaStreamDestroy(s) emu::Ok()
-#define cudaThreadExchangeStreamCaptureMode(m) emu::Ok()
 #define cudaStreamIsCapturing(s, st) (*(st) = cudaStreamCaptureStatusNone, emu::Ok())
 
 #include "../../notorious-fft_b200/csrc/nfft_plan.cu"
