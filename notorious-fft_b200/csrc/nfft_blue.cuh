@@ -135,8 +135,8 @@ struct Blue {
         for (int q = 0; q < 16 / RHO; ++q) {
             int l, i;
             map<LR>(t, q, l, i);
-            // up to 8 different k: few entries per load, so all roots come from the tables
-            if constexpr (LNS > 3) mul_roots<T, LR, LNS>(tw, i & ((1 << LNS) - 1), v + q * RHO);
+            // up to M = 64 there are at most 4 different k: few entries per load
+            if constexpr (LNS > 0 && LOGM > 6) mul_roots<T, LR, LNS>(tw, i & ((1 << LNS) - 1), v + q * RHO);
             else if constexpr (LNS > 0) mul_table<T, LR, LNS>(tw, i & ((1 << LNS) - 1), v + q * RHO);
             dft_radix<T, RHO>(v + q * RHO);
         }
