@@ -283,7 +283,8 @@ int notorious_fft_tune_lookup_plan(int kind, int N, int* log2_radices, int max_p
 /* The schedule an aux runs on one axis (0 = slowest, -1 = last): the pass
  * radices (log2) of the axis's power-of-two inner FFT and the thread count
  * (log2, 0 = the default rule) of its pass kernels.  Returns the pass count,
- * 0 for a Bluestein axis, -1 on error. */
+ * 0 for a Bluestein axis, -1 on error.  (The float library runs the two default
+ * passes of a 16384-point axis as one sweep in calls of up to 2^25 points.) */
 int notorious_fft_aux_schedule(const notorious_fft_aux* a, int axis, int* log2_radices, int max_passes,
                                int* log2_threads);
 

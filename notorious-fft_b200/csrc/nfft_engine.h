@@ -98,6 +98,8 @@ struct AxisPlan {
     int logn = 0;
     // power-of-two inner complex FFT (length n for dft, n/2 for the real families)
     FftSchedule fft_contig, fft_strided;
+    // plain calls run the schedule's passes as one cluster pass
+    bool cluster_contig = false, cluster_strided = false;
     // Bluestein (complex family, n not a power of two)
     int logM = 0;
     cplx_t* chirp = nullptr;   // e^{-i pi k^2/n}, k < n

@@ -503,7 +503,7 @@ bool run_pass(const DeviceCtx* c, const View& src, const View& dst, int logL, in
         if (op.logt && lean_available(logR, op.logt, ci, co, ldop, stop)) logT = op.logt;   // tuned
         // tiles that leave one CTA per SM: the same tile over a cluster (a tuned
         // thread count selects the plain kernel where there is one)
-        if (ldop == LD_C && stop == ST_C && (!op.logt || logR > 13) && cluster_available(logR, ci, co))
+        if (ldop == LD_C && stop == ST_C && !op.logt && cluster_available(logR, ci, co))
             return launch_cluster(a, ci, co, s);
         // the repacking first pass of DCT-3 / DST-3 and invrealdft pairs lines of
         // one transform in its tile: no more lines per tile than per transform
@@ -553,16 +553,17 @@ static bool run_pow2_axis(notorious_fft_plan* p, const DeviceCtx* c, const AxisP
                           const OpSpec& op, cudaStream_t s) {
     const int logL = ax.fft_contig.logL;
     const bool strided = !(src.estride == 1 && dst.estride == 1);
-    // one-pass schedules that only the cluster kernels run (build_axis) serve the
-    // plain form; everything else keeps the schedule without them
     FftSchedule sch = strided ? ax.fft_strided : ax.fft_contig;
-    const bool plain = op.ld == LD_C && op.st == ST_C && !op.tc && !lean_disabled();
-    // (contiguous ones up to 2^25 points: a bigger batch streams faster in two plain
-    // passes.  B200, float 2^14, plain launches of two passes -> one sweep: 1001 lines
-    // 98 -> 90 us, 2000 179 -> 175, 3000 259 -> 261, 4096 350 -> 365, 8192 685 -> 735)
-    const bool big = !strided && (src.lines() << logL) > (1ll << 25);
-    if ((!plain || big) && sch.npass == 1 && sch.plog[0] > (strided ? 13 - log_jmin() : 13))
-        sch = make_schedule(logL, strided);
+    // plain passes that a cluster runs as one (build_axis); contiguous ones up to
+    // 2^25 points: a bigger batch streams faster in two.  B200, float 2^14, plain
+    // launches of two passes -> one sweep: 1001 lines 98 -> 90 us, 2000 179 -> 175,
+    // 3000 259 -> 261, 4096 350 -> 365, 8192 685 -> 735
+    if ((strided ? ax.cluster_strided : ax.cluster_contig && (src.lines() << logL) <= (1ll << 25)) && op.ld == LD_C &&
+        op.st == ST_C && !op.tc && !lean_disabled()) {
+        sch.npass = 1;
+        sch.plog[0] = sch.tile[0] = logL;
+        split_sub(logL, &sch.nsub[0], sch.sub[0]);
+    }
     const long long L = 1ll << logL;
     const int np = sch.npass;
     // a paired operator on a strided axis runs in one pass where the kernel with
@@ -785,17 +786,11 @@ static bool build_axis(notorious_fft_plan* p, const DeviceCtx* c, AxisPlan& ax, 
         int logL = (family == FAM_DFT) ? ax.logn : std::max(0, ax.logn - 1);
         ax.fft_contig = make_schedule(logL, false, max_tile);
         ax.fft_strided = make_schedule(logL, true, max_tile);
+        // one pass instead of several where a cluster's tile holds the line (float:
+        // 2^14 contiguous, 2^11 strided): run_pow2_axis
         if (family == FAM_DFT && max_tile == 13) {
-            // one pass instead of two where a cluster's tile holds the line (float:
-            // 2^14 contiguous, 2^11 strided): run_pow2_axis
-            auto one_pass = [&](FftSchedule& f, int ci) {
-                if (f.npass == 1 || !cluster_available(logL, ci, ci)) return;
-                f.npass = 1;
-                f.plog[0] = f.tile[0] = logL;
-                split_sub(logL, &f.nsub[0], f.sub[0]);
-            };
-            one_pass(ax.fft_contig, 0);
-            one_pass(ax.fft_strided, 1);
+            ax.cluster_contig = ax.fft_contig.npass > 1 && cluster_available(logL, 0, 0);
+            ax.cluster_strided = ax.fft_strided.npass > 1 && cluster_available(logL, 1, 1);
         }
         // standalone plans: an autotuner trial, else the tune cache's split and
         // thread count for (family, n) on this GPU (a split this build cannot
@@ -813,10 +808,12 @@ static bool build_axis(notorious_fft_plan* p, const DeviceCtx* c, AxisPlan& ax, 
             }
             if (have) {
                 FftSchedule t;
-                if (split.empty()) t = ax.fft_contig;
-                else if (!make_split_schedule(logL, split.data(), (int)split.size(), &t)) t = ax.fft_contig;
+                const bool own = !split.empty() && make_split_schedule(logL, split.data(), (int)split.size(), &t);
+                if (!own) t = ax.fft_contig;
                 t.logt = (logt == 7 || logt == 8 || logt == 9) ? logt : 0;
                 ax.fft_contig = t;
+                // (a schedule asked for by its thread count or split is the one that runs)
+                if (t.logt || own) ax.cluster_contig = false;
             }
         }
         return true;
