@@ -77,6 +77,33 @@ NFFT_HD C2<T> table_root(const TwTables<T>* tw, uint32_t q) {
     else return twiddle<T>(tw, (uint64_t)q, LOGP);
 }
 
+// W_{2^logP}^k for a run of k that agree in their low logP - 12 bits: the factor of
+// those bits is made once, each root is one entry of the first table times it, with
+// the roundings of twiddle().  mirror() gives W^{K - k} for a K whose low bits are zero.
+template <typename T>
+struct RootRun {
+    C2<T> low;
+    int logP;
+    bool has;
+    NFFT_HD void start(const TwTables<T>* tw, long long k, int logP_) {
+        logP = logP_;
+        const uint64_t u = (uint64_t)k << (36 - logP);
+        const uint32_t i1 = (uint32_t)(u >> TW_BITS) & (TW_SIZE - 1), i2 = (uint32_t)u & (TW_SIZE - 1);
+        has = i1 || i2;
+        low = i1 ? tw_load<T>(tw, 1, i1) : mkc((T)1, (T)0);
+        if (i2) low = cmul(low, tw_load<T>(tw, 2, i2));
+    }
+    NFFT_HD uint32_t digit(long long k) const { return (uint32_t)(((uint64_t)k << (36 - logP)) >> (2 * TW_BITS)); }
+    NFFT_HD C2<T> at(const TwTables<T>* tw, long long k) const {
+        const C2<T> w = tw_load<T>(tw, 0, digit(k) & (TW_SIZE - 1));
+        return has ? cmul(w, low) : w;
+    }
+    NFFT_HD C2<T> mirror(const TwTables<T>* tw, long long K, long long k) const {
+        const C2<T> w = tw_load<T>(tw, 0, (digit(K) - digit(k)) & (TW_SIZE - 1));
+        return has ? cmulc(w, low) : w;
+    }
+};
+
 // v[m] *= W_{2^(LNS + LR)}^{m k}, m < 2^LR (the internal twiddles of a
 // sub-stage): the roots of m = 1, 2, 3 and of the multiples of 4 from the
 // tables (L1 hits), the others as one product of two of them -- one rounding
@@ -387,20 +414,17 @@ struct Lean {
         if constexpr (WHOLE_COL) {
             mul_table<T, LR, lns>(tw, k, v);
         } else if (k) {
-            // W^{m k} for m < RHO from the root W^k by products (depth <= 4); radix 8
-            // takes W^{4 k} from the table too.  From W^k alone its error grows
-            // with m: as a tree it was 3% above a chain of six products in the
-            // result of a 128- or 512-point transform, as a chain slower; with the
-            // second root it is below both.
+            // W^{m k} for m < RHO from the root W^k: radix 16 by a product tree (depth
+            // 4), radix 8 by a chain (a tree of depth 3 puts the result of a 128- or
+            // 512-point transform 3% further off; W^{4 k} from the table 20% less far,
+            // but its entries lie a cache line apart)
             C2<T> p[16];
             p[1] = table_root<T, lns + LR>(tw, (uint32_t)k);
             if constexpr (RHO == 16) {
                 powers16<T>(p[1], p);
             } else {
-                if constexpr (RHO == 8) p[4] = table_root<T, lns + LR>(tw, (uint32_t)(4 * k));
 #pragma unroll
-                for (int m = 2; m < RHO; ++m)
-                    if (m != 4) p[m] = cmul(p[m & 4 ? 4 : m / 2], p[m & 4 ? m - 4 : m - m / 2]);
+                for (int m = 2; m < RHO; ++m) p[m] = cmul(p[m - 1], p[1]);
             }
 #pragma unroll
             for (int m = 1; m < RHO; ++m) v[m] = cmul(v[m], p[m]);
@@ -576,12 +600,11 @@ NFFT_HD void mirror_unpack_thread(const PassArgs& a, const TwTables<T>* tw, cons
 
 // Paired unpack of whole lines (realdft unpack / DCT-2 post pairs), the items of
 // thread t: an item is the bin pair k, R - k of one line, R the packed spectrum
-// length.  Row tiles: item w is pair w mod (R/2) of line w / (R/2); with
-// R/2 > THREADS a thread walks one line at a time with k stepping by THREADS
-// (twiddles times the exact ratios W_N^THREADS and e^{-i pi THREADS / 2N}; a table
-// root per pair instead is 3% slower at 8192 points), taking a new root from the
-// table after R/512 pairs: the chain of a 256-thread tile, whatever the tile.
-// Otherwise its k is the same on every line and the twiddles are reused.
+// length.  Row tiles: a thread takes the same k of every line of the tile (its
+// twiddles serve them all); with R/2 > THREADS its k steps by THREADS (twiddles times
+// the exact ratios W_N^THREADS and e^{-i pi THREADS / 2N}; a table root per pair
+// instead is 3% slower at 8192 points), with a new root from the table after R/512
+// pairs: the chain of a 256-thread tile, whatever the tile.
 // Column tiles: lines fastest, k stepping by THREADS / J, every root from the tables
 // (the lines of a tile share it).  Bin 0 (with bins M and M/2) goes through unpack_pair.
 template <typename L, typename T, int STORE>
@@ -591,32 +614,46 @@ NFFT_HD void paired_unpack_thread(const PassArgs& a, const TwTables<T>* tw, cons
     constexpr int LOGR = L::LOGR_;
     constexpr int HALF = LOGR == 0 ? 1 : (1 << (LOGR - 1));
     constexpr int ITEMS = L::J * HALF;
-    V ws = V{}, ts = V{};
-    if constexpr (!L::WHOLE_COL && HALF > L::THREADS) {
-        ws = twiddle<T>(tw, (uint64_t)L::THREADS, a.logN);
-        if constexpr (STORE == ST_T2) ts = twiddle<T>(tw, (uint64_t)L::THREADS, a.logN + 2);
-    }
-    V wk = V{}, tk = V{};
-    int prevk = -1;
-    constexpr int CHAIN = HALF < 256 ? 1 : HALF / 256;   // pairs per table root
-    for (int w = t; w < ITEMS; w += L::THREADS) {
-        const int ll = L::WHOLE_COL ? w & (L::J - 1) : w / HALF, k = L::WHOLE_COL ? w / L::J : w & (HALF - 1);
+    auto emit = [&](int ll, int k, V wk, V tk) {
         const LeanLine ln = lines[ll];
-        if (ln.j < 0) continue;
+        if (ln.j < 0) return;
         auto zget = [&](long long r) { return sm[NFFT_SM((lean_idx<L::COLL, LOGR, L::LOGJ>(ll, (int)r)))]; };
-        if (k == 0) {
-            unpack_pair<T, STORE>(a, tw, ln.bout, 0, (long long)(1 << LOGR), zget);
-            continue;
+        if (k == 0) unpack_pair<T, STORE>(a, tw, ln.bout, 0, (long long)(1 << LOGR), zget);
+        else unpack_pair_tw<T, STORE>(a, tw, ln.bout, k, (long long)(1 << LOGR), zget, wk, tk);
+    };
+    auto roots = [&](int k, V& wk, V& tk) {
+        wk = twiddle<T>(tw, (uint64_t)k, a.logN);
+        if constexpr (STORE == ST_T2) tk = twiddle<T>(tw, (uint64_t)k, a.logN + 2);
+    };
+    V wk = V{}, tk = V{};
+    if constexpr (L::WHOLE_COL) {
+        for (int w = t; w < ITEMS; w += L::THREADS) {
+            roots(w / L::J, wk, tk);
+            emit(w & (L::J - 1), w / L::J, wk, tk);
         }
-        if (L::WHOLE_COL || prevk < 0 || k < prevk || (k != prevk && (k / L::THREADS) % CHAIN == 0)) {
-            wk = twiddle<T>(tw, (uint64_t)k, a.logN);
-            if constexpr (STORE == ST_T2) tk = twiddle<T>(tw, (uint64_t)k, a.logN + 2);
-        } else if (k != prevk) {
-            wk = cmul(wk, ws);
-            if constexpr (STORE == ST_T2) tk = cmul(tk, ts);
+    } else {
+        constexpr int STEPS = HALF > L::THREADS ? HALF / L::THREADS : 1;    // pairs of a line per thread
+        constexpr int EVERY = HALF > L::THREADS ? 1 : L::THREADS / HALF;    // lines of a thread
+        constexpr int CHAIN = HALF < 256 ? 1 : HALF / 256;                  // pairs per table root
+        V ws = V{}, ts = V{};
+        if constexpr (STEPS > 1 && CHAIN > 1) {
+            ws = twiddle<T>(tw, (uint64_t)L::THREADS, a.logN);
+            if constexpr (STORE == ST_T2) ts = twiddle<T>(tw, (uint64_t)L::THREADS, a.logN + 2);
         }
-        prevk = k;
-        unpack_pair_tw<T, STORE>(a, tw, ln.bout, k, (long long)(1 << LOGR), zget, wk, tk);
+        // whole in double and for realdft; two at a time for the float DCT-2, whose 64
+        // registers do not hold more (4096 x 4000 all at once: 50 us, so 45)
+        constexpr int UNROLL = sizeof(T) == 8 || STORE == ST_R ? STEPS : 2;
+#pragma unroll UNROLL
+        for (int s = 0; s < STEPS; ++s) {
+            const int k = (t & (HALF - 1)) + s * L::THREADS;
+            if (s % CHAIN == 0 || k == L::THREADS) {   // (bin 0 has no twiddles to go on from)
+                roots(k, wk, tk);
+            } else {
+                wk = cmul(wk, ws);
+                if constexpr (STORE == ST_T2) tk = cmul(tk, ts);
+            }
+            for (int ll = HALF > L::THREADS ? 0 : t / HALF; ll < L::J; ll += EVERY) emit(ll, k, wk, tk);
+        }
     }
 }
 
@@ -678,17 +715,22 @@ NFFT_HD void pair_prepack_thread(const PassArgs& a, const TwTables<T>* tw, C2<T>
     };
     // the two bins of pair k as raw input values: zk, zm (LD_IR), or the reals
     // (x_k, x_{N-k}), (x_{M-k}, x_{M+k}) behind zb_k and zb_{M-k} (LD_T3)
-    auto raw = [&](long long base, long long k, V& u, V& v) {
+    auto raw_k = [&](long long base, long long k) {
         if constexpr (LOAD == LD_IR) {
-            const V* z = (const V*)a.in + base;
-            u = NFFT_GLD(&z[k * es]);
-            v = NFFT_GLD(&z[(M - k) * es]);
+            return NFFT_GLD((const V*)a.in + base + k * es);
         } else {
             const T* x = (const T*)a.in + base;
             const long long iA = a.dst ? N - 1 - k : k, iB = k == 0 ? iA : (a.dst ? k - 1 : N - k);
+            return mkc(NFFT_GLD(&x[iA * es]), NFFT_GLD(&x[iB * es]));
+        }
+    };
+    auto raw_m = [&](long long base, long long k) {
+        if constexpr (LOAD == LD_IR) {
+            return NFFT_GLD((const V*)a.in + base + (M - k) * es);
+        } else {
+            const T* x = (const T*)a.in + base;
             const long long iC = a.dst ? M - 1 + k : M - k, iD = a.dst ? M - 1 - k : M + k;
-            u = mkc(NFFT_GLD(&x[iA * es]), NFFT_GLD(&x[iB * es]));
-            v = mkc(NFFT_GLD(&x[iC * es]), NFFT_GLD(&x[iD * es]));
+            return mkc(NFFT_GLD(&x[iC * es]), NFFT_GLD(&x[iD * es]));
         }
     };
     auto pre = [&](V x, V tq) { return mkc(x.x * tq.x - x.y * tq.y, -x.x * tq.y - x.y * tq.x); };
@@ -698,7 +740,7 @@ NFFT_HD void pair_prepack_thread(const PassArgs& a, const TwTables<T>* tw, C2<T>
         const V od = cmulc(d, w2);
         return cconj(mkc(s2.x - od.y, s2.y + od.x));
     };
-    V u[NI], v[NI], uh = V{}, vh = V{};
+    V u[NI], v[NI], uh = V{};
     // bin M / 2 pairs with itself: one per line (row tiles) or transform
     const bool half = MIR ? self && t < H : t < L::J && lines[t].j >= 0;
 #pragma unroll
@@ -706,30 +748,33 @@ NFFT_HD void pair_prepack_thread(const PassArgs& a, const TwTables<T>* tw, C2<T>
         int lA, rA, lB, rB;
         const long long k = item(q, lA, rA, lB, rB);
         const LeanLine ln = lines[lA];
-        if (ln.j >= 0) raw(ln.bin, k, u[q], v[q]);
-        else u[q] = v[q] = mkc((T)0, (T)0);
+        u[q] = ln.j >= 0 ? raw_k(ln.bin, k) : mkc((T)0, (T)0);
+        v[q] = ln.j >= 0 ? raw_m(ln.bin, k) : mkc((T)0, (T)0);
     }
-    if (half) raw(lines[MIR ? 0 : t].bin, M / 2, uh, vh);
+    if (half) uh = raw_k(lines[MIR ? 0 : t].bin, M / 2);
     // Twiddles from the tables, pair by pair: as products of the thread's first root
     // with exact ones they cost a rounding more (DCT-3 of 8192 points and more, error
-    // up to 4% larger).  Row tiles of short lines have the same k in every pair.
+    // up to 4% larger).  The bins of a thread differ in multiples of D ns (mirror-in
+    // tiles) or THREADS (row tiles), so of each root's table entries only the first
+    // changes (RootRun); row tiles of short lines have the same k in every pair.
     constexpr bool SAME_K = !MIR && !WC && H <= L::THREADS;
+    const int logN = MIR ? a.logN : LOGR + 1;
+    RootRun<T> run_w, run_t;
     V wk = V{}, tk = V{}, tm = V{};
 #pragma unroll
     for (int q = 0; q < NI; ++q) {
         int lA, rA, lB, rB;
         const long long k = item(q, lA, rA, lB, rB);
-        if constexpr (MIR) {
-            wk = twiddle<T>(tw, (uint64_t)k, a.logN);
+        // (a self-paired low line gives way to its high line in the middle)
+        if (q == 0 || (MIR && q == NI / 2 && self)) {
+            run_w.start(tw, k, logN);
+            if constexpr (LOAD == LD_T3) run_t.start(tw, k, logN + 2);
+        }
+        if (q == 0 || !SAME_K) {
+            wk = run_w.at(tw, k);
             if constexpr (LOAD == LD_T3) {
-                tk = twiddle<T>(tw, (uint64_t)k, a.logN + 2);
-                tm = twiddle<T>(tw, (uint64_t)(M - k), a.logN + 2);
-            }
-        } else if (q == 0 || !SAME_K) {
-            wk = table_root<T, LOGR + 1>(tw, (uint32_t)k);
-            if constexpr (LOAD == LD_T3) {
-                tk = table_root<T, LOGR + 3>(tw, (uint32_t)k);
-                if constexpr (WC) tm = table_root<T, LOGR + 3>(tw, (uint32_t)(M - k));
+                tk = run_t.at(tw, k);
+                if constexpr (MIR || WC) tm = run_t.mirror(tw, M, k);
                 else tm = mkc((tk.x - tk.y) * K<T>::r2, -(tk.x + tk.y) * K<T>::r2);
             }
         }
@@ -758,7 +803,6 @@ NFFT_HD void pair_prepack_thread(const PassArgs& a, const TwTables<T>* tw, C2<T>
         else z = cscale(pre(z, mkc(K<T>::c8, -K<T>::s8)), (T)2);
         put(MIR ? 0 : t, R / 2, z);
     }
-    (void)vh;
 }
 
 // One tile of a specialized pass (all threads of the CTA call it; uniform
