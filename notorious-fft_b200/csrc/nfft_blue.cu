@@ -8,9 +8,11 @@ namespace {
 struct BlueEntry {
     void (*fn)(const PassArgs) = nullptr;
     size_t smem = 0;
+    int per_sm = 1;
 };
 template <int LOGM> BlueEntry blue_entry() {
-    return BlueEntry{blue_kernel<real_t, LOGM>, blue_smem_bytes<real_t, LOGM, blue_logt(LOGM), LD_BLUE, ST_BLUE>()};
+    return BlueEntry{blue_kernel<real_t, LOGM>, blue_smem_bytes<real_t, LOGM, blue_logt(LOGM), LD_BLUE, ST_BLUE>(),
+                     lean_min_blocks<real_t, blue_logt(LOGM)>()};
 }
 const BlueEntry* blue_find(int logM) {
     static const BlueEntry tab[] = {blue_entry<4>(), blue_entry<5>(), blue_entry<6>(), blue_entry<7>(), blue_entry<8>(),
@@ -43,7 +45,8 @@ bool launch_blue(PassArgs a, cudaStream_t s) {
     dim3 grid((unsigned)ntiles, 1, 1);
     if (ntiles > 0x7fffffffll) grid = dim3(0x7fffffffu, (unsigned)((ntiles + 0x7fffffffll - 1) / 0x7fffffffll), 1);
     void* args[] = {(void*)&a};
-    return cuda_ok(launch_dependent((const void*)e->fn, grid, 1 << logT, e->smem, args, s), "Bluestein tile kernel launch");
+    return cuda_ok(launch_dependent((const void*)e->fn, grid, 1 << logT, e->smem, args, s, e->per_sm, false),
+                   "Bluestein tile kernel launch");
 }
 
 }  // namespace nfft

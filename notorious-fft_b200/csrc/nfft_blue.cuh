@@ -275,7 +275,6 @@ __global__ void __launch_bounds__(1 << blue_logt(LOGM), (lean_min_blocks<T, blue
 blue_kernel(const PassArgs a) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const long long tile = (long long)blockIdx.x + (long long)blockIdx.y * gridDim.x;
-    pdl_trigger();
     blue_tile<T, LOGM, blue_logt(LOGM), LD_BLUE, ST_BLUE, true>(a, tile, smraw);
 }
 

@@ -55,6 +55,7 @@ bool launch_cluster(PassArgs a, int ci, int co, cudaStream_t s) {
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)e->size;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    // (two CTAs per SM: plain_launch() would keep none of these grids plain)
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};

@@ -195,7 +195,6 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 256 : 512, 2) cluster_kernel(
     const TwTables<T>* tw = (const TwTables<T>*)a.tw;
     const int t = threadIdx.x;
     const int c = (int)cluster_rank();
-    pdl_trigger();
     const long long tile = (long long)blockIdx.x >> LOGC;   // every CTA of the grid has a tile
     if (t < K::J) {
         long long tmp[3];

@@ -210,8 +210,26 @@ bool run_pass(const DeviceCtx* c, const View& src, const View& dst, int logL, in
 View scratch_view(void* ptr, const View& like, long long L, bool strided);
 
 // Kernel launchers (nfft_kernels.cu).  launch_dependent: for kernels whose every
-// CTA calls pdl_wait() before it touches data; counts the launch.
-cudaError_t launch_dependent(const void* fn, dim3 grid, int threads, size_t smem, void** args, cudaStream_t s);
+// CTA calls pdl_wait() before it touches data; counts the launch.  per_sm: resident
+// CTAs per SM; complex_pass: plain complex loads and stores.
+cudaError_t launch_dependent(const void* fn, dim3 grid, int threads, size_t smem, void** args, cudaStream_t s, int per_sm,
+                             bool complex_pass);
+// Whether a grid of `ctas` keeps the plain launch.  Two grids of up to half the
+// places, or one that fills the chip, overlap well: B200, kernels back to back, plain
+// launches -> dependent ones, FP64 1024-point lines on 74 / 148 / 259 / 592 of 592
+// places 1.37 / 1.32 / 1.55 / 1.28 times as fast, FP32 realdft of 64 points on 148 /
+// 518 / 1184 of 1184 places 1.59 / 1.21 / 1.20.  Of a second grid of more than half the places a part is
+// placed early, unevenly.  Where an SM holds four or eight CTAs the real-family and
+// Bluestein kernels lose by that up to four fifths of the places (FP32 666 / 740 /
+// 888 of 1184: realdft 0.81 / 0.81 / 0.94, 1000-point Bluestein 0.81 / 0.80 / 0.91; FP64
+// 333 / 444 of 592: 0.97 / 0.96, 0.97 / 0.94), the complex ones only where it holds eight,
+// up to two thirds (1024-point lines 0.93 / 0.95 / 1.15; of four: FP32 4096 points on 333 /
+// 444 of 592 1.12 / 1.18, FP64 1024 points 1.05 / 1.18).  With one or two CTAs per SM none does.
+constexpr bool plain_launch(long long ctas, int sms, int per_sm, bool complex_pass) {
+    const long long places = (long long)sms * per_sm;
+    if (per_sm <= 2 || 2 * ctas <= places) return false;
+    return complex_pass ? per_sm >= 8 && 3 * ctas < 2 * places : 5 * ctas < 4 * places;
+}
 bool launch_pass(const PassArgs& a, int load_op, int store_op, int log_tile, long long ntiles, cudaStream_t s);
 bool launch_unpack(const PassArgs& a, int store_op, const cplx_t* Z, long long zdist, long long nlines, cudaStream_t s);
 bool launch_tiny(const real_t* x, real_t* y, long long howmany, long long inner, long long idist, long long odist,
@@ -220,7 +238,7 @@ bool launch_init_tables(TwTables<real_t>* tw, cudaStream_t s);
 bool launch_chirp(cplx_t* chirp, cplx_t* bwrap, long long n, long long M, cudaStream_t s);
 // post[q] = e^{-i pi q / 2n}, q < n (FP64 sincospi)
 bool launch_post(cplx_t* post, long long n, cudaStream_t s);
-bool set_kernel_attributes();
+bool set_kernel_attributes(int sms);
 
 // Persistent queue kernel (nfft_queue_kernel.cu)
 struct QueueArgs;

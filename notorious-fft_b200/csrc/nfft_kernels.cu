@@ -3,6 +3,7 @@
 // tables from FP64 sincospi; Bluestein chirp from exact k^2 mod 2n).
 #include "nfft_blue.h"
 #include "nfft_cluster.h"
+#include "nfft_lean.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -14,6 +15,7 @@ namespace nfft {
 static std::atomic<long long> g_launches{0};
 long long launch_count() { return g_launches.load(); }
 void note_launch() { g_launches++; }
+static std::atomic<int> g_sms{148};   // of the GPUs of this node (all alike)
 
 // Generic pass kernels (nfft_pass_slice.cuh, compiled in slices).
 using PassFn = void (*)(const PassArgs);
@@ -77,20 +79,10 @@ bool lean_available(int logR, int logT, int ci, int co, int ld, int st) {
 }
 
 // Launch as a dependent of the stream's previous kernel (pdl_wait), so that the
-// launch and the line set-up overlap the predecessor's last CTAs.  B200, plain
-// launches -> these: FP64 4096 x 256 both ways 20.5 -> 17.5 us, 262144 x 4 both
-// ways 47 -> 36, realdft + invrealdft 32768 x 100 66 -> 55, 65536 x 1000 707 -> 678;
-// FP32 65536 x 1 12.3 -> 9.7.
-// Grids that fill between a quarter and half of the chip's CTA places keep
-// the plain launch: on an idle chip the scheduler spreads them over the SMs, but
-// beside a predecessor of that size the early CTAs take second places on some SMs
-// while others idle (FP64 DCT-2 + DCT-3 4096 x 230, 115 of 296 places: 26.6 us plain,
-// 30.7 dependent; FP32 256 x 256 x 33, 264 of 592: 47 and 63; from 320 of 592 up --
-// FP64 2048 x 64 x 5 22.5 and 18.8 -- and down from 128 of 592 they win).
-cudaError_t launch_dependent(const void* fn, dim3 grid, int threads, size_t smem, void** args, cudaStream_t s) {
-    // CTA places: the register budgets of lean_min_blocks on 148 SMs
-    const unsigned long long places = 148ull * (unsigned)std::max(1, (sizeof(real_t) == 8 ? 512 : 1024) / threads);
-    const unsigned long long ctas = (unsigned long long)grid.x * grid.y;
+// launch and the line set-up overlap the predecessor's last CTAs, unless
+// plain_launch() says otherwise.
+cudaError_t launch_dependent(const void* fn, dim3 grid, int threads, size_t smem, void** args, cudaStream_t s, int per_sm,
+                             bool complex_pass) {
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
@@ -100,9 +92,22 @@ cudaError_t launch_dependent(const void* fn, dim3 grid, int threads, size_t smem
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cfg.attrs = &at;
-    cfg.numAttrs = ctas * 4 > places && ctas * 2 < places ? 0 : 1;
+    cfg.numAttrs = plain_launch((long long)grid.x * grid.y, g_sms.load(std::memory_order_relaxed), per_sm, complex_pass) ? 0 : 1;
     g_launches++;
     return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
+// Resident CTAs per SM of a kernel without a stated register budget.
+static int resident_ctas(std::atomic<int>& cache, const void* fn, int threads, size_t smem) {
+    int n = cache.load(std::memory_order_relaxed);
+    if (!n) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, threads, smem) != cudaSuccess) {
+            cudaGetLastError();
+            n = 1;
+        }
+        cache.store(n = std::max(n, 1), std::memory_order_relaxed);
+    }
+    return n;
 }
 
 bool launch_lean(const PassArgs& a, int logT, int ci, int co, int ld, int st, long long ntiles, cudaStream_t s) {
@@ -116,10 +121,13 @@ bool launch_lean(const PassArgs& a, int logT, int ci, int co, int ld, int st, lo
     if (ntiles <= 0x7fffffffll) grid = dim3((unsigned)ntiles, 1, 1);
     else grid = dim3(0x7fffffffu, (unsigned)((ntiles + 0x7fffffffll - 1) / 0x7fffffffll), 1);
     void* args[] = {(void*)&a};
-    return cuda_ok(launch_dependent(e->fn, grid, e->threads, e->smem, args, s), "specialized pass kernel launch");
+    const int per_sm = logT == 7 ? lean_min_blocks<real_t, 7>() : logT == 8 ? lean_min_blocks<real_t, 8>() : lean_min_blocks<real_t, 9>();
+    return cuda_ok(launch_dependent(e->fn, grid, e->threads, e->smem, args, s, per_sm, ld == LD_C && st == ST_C),
+                   "specialized pass kernel launch");
 }
 
-bool set_kernel_attributes() {
+bool set_kernel_attributes(int sms) {
+    g_sms.store(sms, std::memory_order_relaxed);
     if (!blue_set_attributes() || !cluster_set_attributes()) return false;
     for (auto& kv : lean_registry().entries) {
         if (!cuda_ok(cudaFuncSetAttribute(kv.second.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kv.second.smem),
@@ -155,7 +163,10 @@ bool launch_pass(const PassArgs& a, int load_op, int store_op, int log_tile, lon
         grid = dim3(0x7fffffffu, (unsigned)gy, 1);
     }
     void* args[] = {(void*)&a};
-    return cuda_ok(launch_dependent((const void*)f, grid, threads, pass_smem_bytes<real_t>(log_tile), args, s),
+    const size_t smem = pass_smem_bytes<real_t>(log_tile);
+    static std::atomic<int> resident[2][NLOAD][NSTORE];
+    const int per_sm = resident_ctas(resident[log_tile == 13][load_op][store_op], (const void*)f, threads, smem);
+    return cuda_ok(launch_dependent((const void*)f, grid, threads, smem, args, s, per_sm, load_op == LD_C && store_op == ST_C),
                    "pass kernel launch");
 }
 
@@ -168,7 +179,9 @@ bool launch_unpack(const PassArgs& a, int store_op, const cplx_t* Z, long long z
     if (blocks < 1) blocks = 1;
     void* args[] = {(void*)&a, (void*)&Z, (void*)&zdist, (void*)&nlines};
     const void* f = store_op == ST_R ? (const void*)unpack_kernel<real_t, ST_R> : (const void*)unpack_kernel<real_t, ST_T2>;
-    return cuda_ok(launch_dependent(f, dim3((unsigned)blocks, 1, 1), threads, 0, args, s), "unpack kernel launch");
+    static std::atomic<int> resident[2];
+    const int per_sm = resident_ctas(resident[store_op == ST_R], f, threads, 0);
+    return cuda_ok(launch_dependent(f, dim3((unsigned)blocks, 1, 1), threads, 0, args, s, per_sm, false), "unpack kernel launch");
 }
 
 bool launch_tiny(const real_t* x, real_t* y, long long howmany, long long inner, long long idist, long long odist,

@@ -640,9 +640,11 @@ NFFT_HD void paired_unpack_thread(const PassArgs& a, const TwTables<T>* tw, cons
             ws = twiddle<T>(tw, (uint64_t)L::THREADS, a.logN);
             if constexpr (STORE == ST_T2) ts = twiddle<T>(tw, (uint64_t)L::THREADS, a.logN + 2);
         }
-        // whole in double and for realdft; two at a time for the float DCT-2, whose 64
-        // registers do not hold more (4096 x 4000 all at once: 50 us, so 45)
-        constexpr int UNROLL = sizeof(T) == 8 || STORE == ST_R ? STEPS : 2;
+        // whole for realdft (FP64 8192 x 1000 38.9 -> 35.4 us, one pair at a time 37.3), two
+        // pairs at a time for the longer code of DCT-2: whole, it does not fit the float
+        // kernel's 64 registers (4096 x 4000 50 us, 45 so), and calls that alternate
+        // with DCT-3 fetch it anew (FP64 8192 x 512 both ways 68.2 us, 61.4 so)
+        constexpr int UNROLL = STORE == ST_R ? STEPS : 2;
 #pragma unroll UNROLL
         for (int s = 0; s < STEPS; ++s) {
             const int k = (t & (HALF - 1)) + s * L::THREADS;
@@ -968,7 +970,6 @@ template <typename T, int LOGR, int LOGT, bool COL_IN, bool COL_OUT, int LOAD, i
 __global__ void __launch_bounds__(1 << LOGT, (lean_min_blocks<T, LOGT>()))
 lean_pass_kernel(const PassArgs a) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    pdl_trigger();
     long long tile = (long long)blockIdx.x + (long long)blockIdx.y * gridDim.x;
     if constexpr (LOAD == LD_FILT) tile = lean_batch_inner(a, tile, Lean<T, LOGR, LOGT, COL_IN, COL_OUT, LOAD, STORE>::LOGJ);
     lean_tile<T, LOGR, LOGT, COL_IN, COL_OUT, LOAD, STORE, true>(a, tile, smraw);

@@ -82,7 +82,7 @@ NoallocDevice* noalloc_device(cudaStream_t stream) {
     void* tw = nullptr;
     if (!cuda_ok(cudaGetSymbolAddress(&scratch, g_noalloc_scratch), "cudaGetSymbolAddress(scratch)")) return nullptr;
     if (!cuda_ok(cudaGetSymbolAddress(&tw, g_noalloc_tw), "cudaGetSymbolAddress(twiddle tables)")) return nullptr;
-    if (!set_kernel_attributes()) return nullptr;
+    if (!set_kernel_attributes(sms)) return nullptr;
     if (!launch_init_tables((TwTables<real_t>*)tw, 0)) return nullptr;
     if (!cuda_ok(cudaStreamSynchronize(0), "twiddle table set-up")) return nullptr;
     d.scratch = (cplx_t*)scratch;

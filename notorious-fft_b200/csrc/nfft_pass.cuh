@@ -613,7 +613,6 @@ template <typename T, int LOG_TILE, int LOAD, int STORE>
 __global__ void __launch_bounds__((1 << LOG_TILE) / 16)
 pass_kernel(const PassArgs a) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    pdl_trigger();
     pass_tile<T, LOG_TILE, LOAD, STORE, true>(a, (long long)blockIdx.x + (long long)blockIdx.y * gridDim.x, smraw);
 }
 
@@ -656,7 +655,6 @@ __global__ void unpack_kernel(const PassArgs a, const C2<T>* Z, long long zdist,
     const long long M = a.N / 2;
     const long long per = M >= 2 ? M / 2 : 1;
     const long long total = per * nlines;
-    pdl_trigger();
     pdl_wait();
     for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (long long)gridDim.x * blockDim.x)
         unpack_item<T, STORE>(a, tw, Z, zdist, w);

@@ -66,7 +66,7 @@ DeviceCtx* device_ctx(int device) {
     c.l2_bytes = (size_t)prop.l2CacheSize;
     if (!cuda_ok(cudaMalloc((void**)&c.tw, sizeof(TwTables<real_t>)), "cudaMalloc(twiddle tables)")) return nullptr;
     if (!launch_init_tables(c.tw, 0)) return nullptr;
-    if (!set_kernel_attributes()) return nullptr;
+    if (!set_kernel_attributes(c.sm_count)) return nullptr;
     if (!cuda_ok(cudaDeviceSynchronize(), "twiddle table init")) return nullptr;
     c.ready = true;
     if (prev >= 0 && prev != device) cudaSetDevice(prev);

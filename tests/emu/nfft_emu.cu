@@ -358,7 +358,7 @@ bool launch_chirp(cplx_t* chirp, cplx_t* bwrap, long long n, long long M, cudaSt
     return true;
 }
 
-bool set_kernel_attributes() { return true; }
+bool set_kernel_attributes(int) { return true; }
 
 // ---- specialized (lean) pass kernels: the kernel body of nfft_lean.cuh, with
 // every phase run for all threads before the next (its __syncthreads points)
