@@ -12,11 +12,12 @@
 // half of the padded input is zero and the upper half of the output is not
 // wanted: both radix-16 end stages touch 8 points of 16.
 //
-// Bound: the FP64 pipe and the exchanges (two M-point FFTs, M >= 2n, per n
-// points of traffic), so tiles are the smallest that hold a line -- 2048 points
-// and 128 threads up to M = 2048, four (FP64) or eight (FP32) CTAs per SM to
-// overlap one tile's loads with another's arithmetic.
-// B200, general kernel -> this one: FP64 1000 x 2000 150 -> 56 us, 300 x 5001
+// Bound: the SM's L1 / shared-memory data path (84% busy in double, 93% in float, at
+// 1000 points; FP64 pipe 38%, DRAM 13%): two M-point FFTs, M >= 2n, with their
+// exchanges and root loads per n points of traffic.  So tiles are the smallest that
+// hold a line -- 2048 points and 128 threads up to M = 2048, four (FP64) or eight (FP32)
+// CTAs per SM to overlap one tile's loads with another's arithmetic.
+// B200, general kernel -> this one: FP64 1000 x 2000 160 -> 58 us, 300 x 5001
 // 174 -> 55 us, 3000 x 500 191 -> 76 us, 230 x 7 33 -> 7 us; FP32 17 x 219837
 // 210 -> 45 us, 500 x 4000 84 -> 29 us.
 #pragma once

@@ -16,8 +16,9 @@
 // 16/C consecutive points (rows) or J consecutive lines (columns).
 //
 // Pairs (C = 2) are what the library runs: half of the points cross, well below
-// what distributed shared memory moves (about 26 bytes per ns and SM).  Bound: FP64 pipe
-// and shared memory in double, HBM and latency in float.  B200, the plain kernels
+// what distributed shared memory moves (about 26 bytes per ns and SM).  Bound: the
+// latency of a tile's phases (two tiles per SM; L1 / shared-memory data path 52 - 57%
+// busy, FP64 pipe 25 - 33%, DRAM 28 - 39%; loads and barriers are the stalls).  B200, the plain kernels
 // (one CTA per SM, or two passes) -> these: FP64 8192 x 2000 165 -> 147 us, x 100
 // 11.6 -> 11.3, 2048 x 2048 72 -> 66, 16 of 1024 x 1024 250 -> 225, 7 of 1024 x 128
 // 18.5 -> 16; FP32 16384 x 1001 95 -> 90, 3 of 2048 x 2048 123 -> 112, 10 of

@@ -108,7 +108,7 @@ struct RootRun {
 // sub-stage): the roots of m = 1, 2, 3 and of the multiples of 4 from the
 // tables (L1 hits), the others as one product of two of them -- one rounding
 // more than a lookup, where a tree from the first root alone has up to four.
-// Reading all of them is slower (Bluestein FP64 1000 x 2000: 84 us, 56 us so).
+// Reading all of them is slower (Bluestein FP64 1000 x 2000: 84 us, 58 us so).
 // The plain passes keep the tree: their tiles are bound by L1 as much as by HBM
 // (B200, FP64 4096 x 256 both ways 20.5 us with the tree, 24.6 with these loads;
 // FP32 8192 x 2000 79 and 92; radices below 16 alone, FP64 1024 x 1024 x 16 258
